@@ -524,13 +524,19 @@ def main():
     tile_kernel, tile_rows, tile_ms = sv.tiles()
     edge_rows, edge_ms = sv.edge_tiles()
     rc_plan = sv.recompute_plan()
+    resident = sv.resident()
     launch_form, launch_direct_ms, launch_graph_ms = sv.launch_form(1)
     stepping, stepping_ms = sv.stepping()
     achieved = bytes_step / step_s / 1e9
     tr = traffic_from_profile()
+    if resident:  # the wave's state stays in shared memory: the step's bytes are what a streaming step would move
+        bytes_step, wave, tr = bytes_single, resident, None
+        achieved = bytes_step / step_s / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "traffic": tr * wave if (tr and a.workload in ("mcs", "mcs-f16")) else None,
-            "kernel": ("one time step of all shots of a wave, run as two-step passes: "
+            "kernel": (f"one time step of the {resident} shots of a k_resident launch (whole time loop in one launch, "
+                       "state in shared memory; the bytes are those of a streaming step)") if resident else
+                      ("one time step of all shots of a wave, run as two-step passes: "
                        + ("k_step2s_interior" if tile_kernel == 2 else "k_step2_interior")
                        + f" (model-row interior, two steps per sweep, {tile_rows}-row tiles) beside k_step_strip + "
                        "k_step_bottom + k_step_interior (single-step lists, twice per pass)") if tile_kernel else
@@ -655,6 +661,7 @@ def main():
                            "tile_edge_rows": edge_rows,
                            "tuner_ms_per_pass": {f"{k}/{r}": v for (k, r), v in tile_ms.items()},
                            "tuner_edge_ms_per_pass": {str(k): v for k, v in edge_ms.items()},
+                           "resident_shots_per_launch": resident,
                            "recompute_segment_steps": rc_plan[0], "recompute_segments": rc_plan[1],
                            "launch": {"form": launch_form, "direct_ms": launch_direct_ms,
                                       "graph_replay_ms": launch_graph_ms},

@@ -372,6 +372,15 @@ class Survey:
         N.check(N.load().fwi_survey_two_step_bytes(self.handle, C.byref(a), C.byref(t)))
         return a.value, t.value
 
+    def resident(self):
+        """Shots whose whole time loop one launch runs with their state in
+        shared memory (the first wave's), 0 where the survey runs the streaming
+        kernels.  tuning(), tiles(), edge_tiles() and stepping() describe the
+        streaming kernels' plan for the same shots either way."""
+        n = C.c_int(0)
+        N.check(N.load().fwi_survey_resident(self.handle, C.byref(n)))
+        return n.value
+
     def tuning(self):
         w, b = C.c_int(0), C.c_int(0)
         N.check(N.load().fwi_survey_tuning(self.handle, C.byref(w), C.byref(b)))

@@ -23,6 +23,7 @@
 #include "fwi_gb300.h"
 #include "fwi_internal.cuh"
 #include "fwi_lists.h"
+#include "fwi_resident.cuh"
 
 namespace fwi {
 cudaError_t launch_step2(int acc, int mode, int var, const StepParams& pf, cudaStream_t st);
@@ -110,6 +111,7 @@ struct LibState {
     // the last survey tuned in this process (the tuner's default before)
     int tile_var = 1, tile_band = TWO_STEP_BAND, tile_eband = 0;
     long long launches = 0;
+    ResDevice res_dev;  // limits of the resident kernel's planner
     std::recursive_mutex mu;
 };
 LibState& L() {
@@ -266,6 +268,17 @@ struct ShotState {
     DBuf ckpt;     // forward-state checkpoints when recomputing
     Layout lay{};
     size_t field_bytes = 0, snap_bytes = 0;
+    // resident waves: the snapshots and the imaging accumulator only
+    int alloc_images(const Layout& l, int nsnap_blocks, int grad_form) {
+        lay = l;
+        snap_bytes = (size_t)nsnap_blocks * l.ny * l.pitch * 4;
+        TRY(snaps.ensure(snap_bytes));
+        TRY(k.ensure(image_bytes(l, grad_form)));
+        return FWI_OK;
+    }
+    static size_t image_bytes(const Layout& l, int grad_form) {
+        return (size_t)l.ny * l.pitch * (grad_form == FWI_GRAD_F64 ? 8 : 4);
+    }
     // the seven fields of a checkpointed state (the state is in wavefield pair 0
     // at every checkpoint): pa, pb, phx, chx, phy, phy2, chy
     void* state(int i) {
@@ -614,12 +627,84 @@ int run_time_loop(int acc, int mode, int nt, int store_snap, int nt_store, bool 
     return run_range(acc, mode, 2, nt, [&](int k) { return sn[k]; }, ps, tw, st, st2);
 }
 
+// A resident launch's plan on the device, for a group of shots; the outboxes
+// and c2 are shared by launches that follow one another on a stream.
+struct ResDev {
+    ResPlan plan;
+    DBuf tiles, shots[2], src, rec, rows;  // shots: forward, adjoint
+};
+
+int res_upload(ResDev& r, cudaStream_t st) {
+    TRY(upload(r.tiles, r.plan.tiles, st));
+    TRY(upload(r.src, r.plan.src, st));
+    TRY(upload(r.rec, r.plan.rec, st));
+    TRY(upload(r.rows, r.plan.rows, st));
+    return FWI_OK;
+}
+
+ResParams res_params(const ResDev& r, int mode, int acc, float dt, float d, int nt, int store_snap, int nt_store,
+                     int grad_form, const DBuf& fA, const DBuf& fB, const DBuf& out, const DBuf& c2g, int* err) {
+    const StepParams b = base_params(acc, dt, store_snap, FWI_SNAP_F32, grad_form, nullptr, nullptr);
+    ResParams p{};
+    p.tiles = r.tiles.as<ResTile>();
+    p.shots = r.shots[mode].as<ResShot>();
+    p.src = r.src.as<ResSrc>();
+    p.rec = r.rec.as<ResRec>();
+    p.rows = r.rows.as<int>();
+    p.out = out.as<uint2>();
+    p.c2g = c2g.as<float>();
+    p.err = err;
+    p.fA = fA.as<float>();
+    p.fB = fB.as<float>();
+    p.nt = p.steps = nt;
+    p.store_snap = store_snap;
+    p.nt_store = nt_store;
+    p.record = mode == 0;
+    p.grad_form = grad_form;
+    p.dt = dt;
+    p.rdt = b.rdt;
+    p.ss = b.ss;
+    p.dt2 = dt * dt;
+    p.d2 = d * d;
+    for (int i = 0; i <= MAXR; ++i) {
+        p.c1[i] = b.c1[i];
+        p.c2[i] = b.c2[i];
+    }
+    return p;
+}
+
+// One resident launch: its outboxes cleared (their words carry step numbers
+// of the launch), then the kernel.
+int res_launch(const ResDev& r, int acc, int mode, const ResParams& p, cudaStream_t st) {
+    CK(cudaMemsetAsync(p.out, 0, r.plan.out_elems * sizeof(uint2), st));
+    LK(launch_resident(acc, mode, p, (int)r.plan.tiles.size(), r.plan.smem, st));
+    return FWI_OK;
+}
+
+// Whether the blocks of a plan are resident together on this device.
+int res_fits(const ResPlan& p, int acc, bool* ok) {
+    int blocks = 0;
+    CK(resident_blocks(acc, p.smem, &blocks));
+    *ok = (long long)blocks * L().res_dev.sms >= (long long)p.tiles.size();
+    return FWI_OK;
+}
+
+int res_error(int err) {
+    return err ? fail(FWI_ERR_CUDA, "the resident kernel gave up waiting for a neighbouring tile") : FWI_OK;
+}
+
 // ---------------------------------------------------------------------------
 // single-shot drop-in state (buffers kept between calls)
 // ---------------------------------------------------------------------------
 
 struct Single {
     ShotState sh;
+    // resident launch: the grid's cut (kept for the last grid), its lists and buffers
+    int cut_key[4] = {0, 0, 0, 0};  // ny, nx, acc, dpml
+    bool cut_ok = false;
+    ResCuts cuts;
+    std::unique_ptr<ResDev> res;
+    DBuf res_out, res_c2, res_err;
     DBuf d_ctmp, d_srcv, d_rec, d_items_m, d_items_b, d_src, d_recs, d_shot, d_fA, d_fB, d_stage, d_flag;
     DBuf d_items_f, d_items_l;  // two-step tiles; single-step interior items beside them
 };
@@ -644,6 +729,22 @@ struct BatchPlan {
 BatchPlan& batch_plan() {
     static BatchPlan b;
     return b;
+}
+
+// The resident plan of the drop-in solver's shot; *ok: whether it fits.
+int single_resident(Single& sg, const ShotGeom& geo, const Layout& l, int dpml, bool* ok) {
+    const int key[4] = {l.ny, l.nx, l.acc, dpml};
+    const std::vector<const Layout*> lays{&l};
+    if (std::memcmp(key, sg.cut_key, sizeof key)) {
+        sg.cut_ok = res_cuts(lays, L().res_dev, sg.cuts);
+        std::memcpy(sg.cut_key, key, sizeof key);
+    }
+    *ok = sg.cut_ok;
+    if (!*ok) return FWI_OK;
+    if (!sg.res) sg.res.reset(new ResDev());
+    *ok = res_plan({&geo}, lays, sg.cuts, L().res_dev, sg.res->plan);
+    if (*ok) TRY(res_fits(sg.res->plan, l.acc, ok));
+    return FWI_OK;
 }
 
 int check_nonfinite(const float* dptr, size_t n, DBuf& flag, cudaStream_t st, const char* what) {
@@ -710,6 +811,14 @@ int fwi_init(int device) {
     for (auto& e : L().ev2)
         if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(configure_step_kernels());
+    CK(configure_resident());
+    {
+        int sms = 0, sm = 0, blk = 0;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        CK(cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+        CK(cudaDeviceGetAttribute(&blk, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+        L().res_dev = ResDevice{sms, (size_t)sm, (size_t)blk};
+    }
     L().device = device;
     L().init = true;
     return FWI_OK;
@@ -804,14 +913,21 @@ int fwi_solver_acoustic_ss(const int* rank, const int* iprop_, const int* NumSou
     Single& sg = single();
     cudaStream_t st = stream();
     const int nsnap_blocks = nt_store + 1;
-    TRY(sg.sh.alloc(l, (iprop == 1 || iprop == 2) ? nsnap_blocks : 1, FWI_SNAP_F32, FWI_GRAD_F32));
-    TRY(sg.sh.zero_state(st));
+    bool resident = false;
+    TRY(single_resident(sg, geo, l, dpml, &resident));
+    if (resident) {
+        TRY(sg.sh.alloc_images(l, (iprop == 1 || iprop == 2) ? nsnap_blocks : 1, FWI_GRAD_F32));
+    } else {
+        TRY(sg.sh.alloc(l, (iprop == 1 || iprop == 2) ? nsnap_blocks : 1, FWI_SNAP_F32, FWI_GRAD_F32));
+        TRY(sg.sh.zero_state(st));
+    }
 
     // model -> c2
     TRY(sg.d_ctmp.ensure((size_t)ny * nx * sizeof(float)));
     CK(cudaMemcpyAsync(sg.d_ctmp.p, ctmp, (size_t)ny * nx * sizeof(float), cudaMemcpyHostToDevice, st));
-    LK(launch_build_c2(sg.sh.c2.as<float>(), l.nyt, l.pitch, l.off, l.dn, ny, nx, sg.d_ctmp.as<float>(), ny, 0, 0,
-                       dt * dt, d * d, st));
+    if (!resident)
+        LK(launch_build_c2(sg.sh.c2.as<float>(), l.nyt, l.pitch, l.off, l.dn, ny, nx, sg.d_ctmp.as<float>(), ny, 0, 0,
+                           dt * dt, d * d, st));
     std::vector<float> fA, fB;
     pml_factors(acc, dpml, dt, d, fA, fB);
     TRY(upload(sg.d_fA, fA, st));
@@ -833,46 +949,72 @@ int fwi_solver_acoustic_ss(const int* rank, const int* iprop_, const int* NumSou
         LK(launch_fields_io(sg.d_stage.as<float>(), sg.sh.snaps.as<float>(), ny, nx, l.pitch, off_dn, nsnap_blocks, 1,
                             st));
         CK(cudaMemsetAsync(sg.sh.k.p, 0, (size_t)ny * l.pitch * sizeof(float), st));
-        TRY(sg.d_ctmp.ensure((size_t)ny * nx * sizeof(float)));
-        CK(cudaMemcpyAsync(sg.d_ctmp.p, kernel, (size_t)ny * nx * sizeof(float), cudaMemcpyHostToDevice, st));
-        LK(launch_kernel_io(sg.sh.k.as<float>(), sg.d_ctmp.as<float>(), ny, nx, l.pitch, off_dn, 1, st));
+        CK(cudaMemcpyAsync(sg.d_stage.p, kernel, (size_t)ny * nx * sizeof(float), cudaMemcpyHostToDevice, st));
+        LK(launch_kernel_io(sg.sh.k.as<float>(), sg.d_stage.as<float>(), ny, nx, l.pitch, off_dn, 1, st));
     }
 
-    // work lists (the adjoint injects at the receivers)
-    std::vector<ShotGeom> geoms{geo};
-    std::vector<Layout> lays{l};
-    Lists lists = build_lists(geoms, lays, 64, L().tile_band, L().tile_eband);
     const bool adj = (iprop == 2);
-    TRY(upload(sg.d_items_m, adj ? lists.int_adj : lists.int_fwd, st));
-    TRY(upload(sg.d_items_b, adj ? lists.bnd_adj : lists.bnd_fwd, st));
-    TRY(upload(sg.d_items_f, adj ? lists.fus_adj : lists.fus_fwd, st));
-    TRY(upload(sg.d_items_l, adj ? lists.lft_adj : lists.lft_fwd, st));
-    TRY(upload(sg.d_src, adj ? lists.src_adj : lists.src_fwd, st));
-    TRY(upload(sg.d_recs, lists.recs, st));
-    std::vector<ShotDev> sd{sg.sh.dev(nt, NumRec, 0, sg.d_srcv.as<float>(), sg.d_rec.as<float>())};
-    TRY(upload(sg.d_shot, sd, st));
+    if (resident) {
+        ResDev& r = *sg.res;
+        TRY(res_upload(r, st));
+        TRY(sg.res_out.ensure(std::max<size_t>(r.plan.out_elems * sizeof(uint2), 16)));
+        TRY(sg.res_c2.ensure(r.plan.c2_elems * sizeof(float)));
+        TRY(sg.res_err.ensure(sizeof(int)));
+        CK(cudaMemsetAsync(sg.res_err.p, 0, sizeof(int), st));
+        ResShot v{};
+        v.model = sg.d_ctmp.as<float>();
+        v.ldv = ny;
+        v.srcv = sg.d_srcv.as<float>();
+        v.rec = sg.d_rec.as<float>();
+        v.snaps = sg.sh.snaps.as<float>();
+        v.k32 = sg.sh.k.as<float>();
+        v.ny = ny;
+        v.nx = nx;
+        v.dn = l.dn;
+        v.off = l.off;
+        v.pitch = l.pitch;
+        const std::vector<ResShot> sv{v};
+        TRY(upload(r.shots[adj], sv, st));
+        ResParams p = res_params(r, adj, acc, dt, d, nt, store_snap, nt_store, FWI_GRAD_F32, sg.d_fA, sg.d_fB,
+                                 sg.res_out, sg.res_c2, sg.res_err.as<int>());
+        p.store = iprop == 1;
+        TRY(res_launch(r, acc, adj, p, st));
+    } else {
+        // work lists (the adjoint injects at the receivers)
+        std::vector<ShotGeom> geoms{geo};
+        std::vector<Layout> lays{l};
+        Lists lists = build_lists(geoms, lays, 64, L().tile_band, L().tile_eband);
+        TRY(upload(sg.d_items_m, adj ? lists.int_adj : lists.int_fwd, st));
+        TRY(upload(sg.d_items_b, adj ? lists.bnd_adj : lists.bnd_fwd, st));
+        TRY(upload(sg.d_items_f, adj ? lists.fus_adj : lists.fus_fwd, st));
+        TRY(upload(sg.d_items_l, adj ? lists.lft_adj : lists.lft_fwd, st));
+        TRY(upload(sg.d_src, adj ? lists.src_adj : lists.src_fwd, st));
+        TRY(upload(sg.d_recs, lists.recs, st));
+        std::vector<ShotDev> sd{sg.sh.dev(nt, NumRec, 0, sg.d_srcv.as<float>(), sg.d_rec.as<float>())};
+        TRY(upload(sg.d_shot, sd, st));
 
-    StepSet ps;
-    ps.pm = base_params(acc, dt, store_snap, FWI_SNAP_F32, FWI_GRAD_F32, sg.d_fA.as<float>(), sg.d_fB.as<float>());
-    ps.pm.items = sg.d_items_m.as<WorkItem>();
-    ps.pm.nitems = (int)(adj ? lists.int_adj.size() : lists.int_fwd.size());
-    ps.pm.shots = sg.d_shot.as<ShotDev>();
-    ps.pm.srcs = sg.d_src.as<SrcEnt>();
-    ps.pm.recs = sg.d_recs.as<RecEnt>();
-    ps.pm.record = adj ? 0 : 1;
-    ps.pb = ps.pm;
-    ps.pb.items = sg.d_items_b.as<WorkItem>();
-    ps.pb.nitems = (int)(adj ? lists.bnd_adj.size() : lists.bnd_fwd.size());
-    ps.pb.nstrip = lists.nstrip;
-    ps.kstrip = lists.kstrip;
-    // pairs of steps as two-step passes (FP32 snapshots: a pass may store or image)
-    const TwoStep tw = two_step_set(ps, adj ? 1 : 0, sg.d_items_f, (int)(adj ? lists.fus_adj : lists.fus_fwd).size(),
-                                    lists.ncore, sg.d_items_l, (int)(adj ? lists.lft_adj : lists.lft_fwd).size(),
-                                    L().tile_var);
-    TRY(run_time_loop(acc, adj ? 1 : 0, nt, store_snap, nt_store, iprop == 1, ps, st, L().aux,
-                      lists.fus_fwd.empty() ? nullptr : &tw));
+        StepSet ps;
+        ps.pm = base_params(acc, dt, store_snap, FWI_SNAP_F32, FWI_GRAD_F32, sg.d_fA.as<float>(), sg.d_fB.as<float>());
+        ps.pm.items = sg.d_items_m.as<WorkItem>();
+        ps.pm.nitems = (int)(adj ? lists.int_adj.size() : lists.int_fwd.size());
+        ps.pm.shots = sg.d_shot.as<ShotDev>();
+        ps.pm.srcs = sg.d_src.as<SrcEnt>();
+        ps.pm.recs = sg.d_recs.as<RecEnt>();
+        ps.pm.record = adj ? 0 : 1;
+        ps.pb = ps.pm;
+        ps.pb.items = sg.d_items_b.as<WorkItem>();
+        ps.pb.nitems = (int)(adj ? lists.bnd_adj.size() : lists.bnd_fwd.size());
+        ps.pb.nstrip = lists.nstrip;
+        ps.kstrip = lists.kstrip;
+        // pairs of steps as two-step passes (FP32 snapshots: a pass may store or image)
+        const TwoStep tw = two_step_set(ps, adj ? 1 : 0, sg.d_items_f, (int)(adj ? lists.fus_adj : lists.fus_fwd).size(),
+                                        lists.ncore, sg.d_items_l, (int)(adj ? lists.lft_adj : lists.lft_fwd).size(),
+                                        L().tile_var);
+        TRY(run_time_loop(acc, adj ? 1 : 0, nt, store_snap, nt_store, iprop == 1, ps, st, L().aux,
+                          lists.fus_fwd.empty() ? nullptr : &tw));
 
-    if (!adj) LK(launch_rec_last(sg.d_rec.as<float>(), nt, NumRec, st));
+        if (!adj) LK(launch_rec_last(sg.d_rec.as<float>(), nt, NumRec, st));
+    }
     // outputs
     if (NumRec > 0)
         CK(cudaMemcpyAsync(Rec_point, sg.d_rec.p, (size_t)nt * NumRec * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -898,7 +1040,10 @@ int fwi_solver_acoustic_ss(const int* rank, const int* iprop_, const int* NumSou
     } else if (NumRec > 0) {
         rc = check_nonfinite(sg.d_rec.as<float>(), (size_t)nt * NumRec, sg.d_flag, st, "Rec_point");
     }
+    int err = 0;
+    if (resident) CK(cudaMemcpyAsync(&err, sg.res_err.p, sizeof err, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    TRY(res_error(err));
     return rc;
 }
 
@@ -1134,6 +1279,12 @@ struct fwi_survey {
     std::vector<std::unique_ptr<WaveDev>> wdev;
     std::vector<float> h_fA, h_fB;
     bool lambda_set = false;
+    // resident waves: plan and device lists of every wave, shared outboxes and
+    // c2; the streaming kernels' plan, made when its tuning is asked for
+    bool resident = false;
+    std::vector<std::unique_ptr<ResDev>> res;
+    DBuf res_out, res_c2;
+    std::unique_ptr<fwi_survey> streaming;
     // checkpointed recomputation: C forward steps per segment, J segments,
     // `slots` snapshot blocks per shot; per block its segment and slot
     int rc_C = 0, rc_J = 0, rc_slots = 0;
@@ -1194,10 +1345,8 @@ int survey_prepare_slots(fwi_survey* s) {
     return FWI_OK;
 }
 
-// Work lists and shot descriptors of every wave for the band height s->band.
-int survey_prepare_waves(fwi_survey* s) {
-    const auto& D = s->desc;
-    cudaStream_t st = stream();
+// Drop every wave's lists, graphs and timings.
+void survey_drop_waves(fwi_survey* s) {
     for (auto& w : s->wdev) {
         for (auto& gexec : w->graph)
             if (gexec) {
@@ -1211,6 +1360,13 @@ int survey_prepare_waves(fwi_survey* s) {
             }
     }
     s->wdev.clear();
+}
+
+// Work lists and shot descriptors of every wave for the band height s->band.
+int survey_prepare_waves(fwi_survey* s) {
+    const auto& D = s->desc;
+    cudaStream_t st = stream();
+    survey_drop_waves(s);
     for (size_t wi = 0; wi < s->waves.size(); ++wi) {
         const auto& w = s->waves[wi];
         std::vector<ShotGeom> g;
@@ -1737,10 +1893,64 @@ int rc_adjoint(fwi_survey* s, size_t wi, StepSet ps, cudaStream_t st, cudaStream
     return run_range(D.acc, 1, k, D.nt, sn_of, ps, pa, st, st2);
 }
 
+// Misfit and adjoint source of a wave's traces (one launch per shot: the
+// shots of a wave need not be consecutive); the observed data may still be on
+// their way (the batch call uploads them beside the forward pass and records
+// obs_ready before it launches a wave); a captured wave waits for that event
+// inside its graph.
+int issue_misfit(fwi_survey* s, size_t wi, cudaStream_t st) {
+    const auto& D = s->desc;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    if (cs == cudaStreamCaptureStatusActive) CK(cudaStreamWaitEvent(st, s->obs_ready, cudaEventWaitExternal));
+    else if (s->obs_pending) CK(cudaStreamWaitEvent(st, s->obs_ready, 0));
+    for (int sh : s->waves[wi]) {
+        const int t0 = s->tr_off[sh], t1 = s->tr_off[sh + 1];
+        if (t1 == t0) continue;
+        LK(launch_misfit(s->d_synth.as<float>() + (size_t)t0 * D.nt, s->d_obs.as<float>() + (size_t)t0 * D.nt,
+                         s->d_adj.as<float>() + (size_t)t0 * D.nt, s->d_mis_tr.as<double>() + t0, D.nt, D.dt,
+                         s->d_tr_off.as<int>(), t1 - t0, 0, nullptr, st));
+    }
+    return FWI_OK;
+}
+
+// A resident wave: forward, misfit, adjoint in one launch each.
+int issue_resident(fwi_survey* s, size_t wi, int step, cudaStream_t st) {
+    const auto& D = s->desc;
+    const auto& w = s->waves[wi];
+    ResDev& r = *s->res[wi];
+    int* err = reinterpret_cast<int*>(s->d_mis_tr.as<double>() + s->ntr);
+    for (size_t k = 0; k < w.size(); ++k) {
+        const Layout& l = s->lays[w[k]];
+        // snapshot block 0: zero, as below; receivers in the top pad stay zero
+        if (step == 1) {
+            CK(cudaMemsetAsync(s->slots[k]->snaps.p, 0, (size_t)l.ny * l.pitch * 4, st));
+            CK(cudaMemsetAsync(s->slots[k]->k.p, 0, ShotState::image_bytes(l, D.grad_form), st));
+        }
+        CK(cudaMemsetAsync(s->d_synth.as<float>() + (size_t)s->tr_off[w[k]] * D.nt, 0,
+                           s->geoms[w[k]].nxR.size() * D.nt * sizeof(float), st));
+    }
+    ResParams p = res_params(r, 0, D.acc, D.dt, D.d, D.nt, D.store_snap, s->nt_store, D.grad_form, s->d_fA, s->d_fB,
+                             s->res_out, s->res_c2, err);
+    p.from_lambda = 1;
+    p.store = step == 1;
+    TRY(res_launch(r, D.acc, 0, p, st));
+    TRY(issue_misfit(s, wi, st));
+    if (step != 1) return FWI_OK;
+    p = res_params(r, 1, D.acc, D.dt, D.d, D.nt, D.store_snap, s->nt_store, D.grad_form, s->d_fA, s->d_fB, s->res_out,
+                   s->res_c2, err);
+    p.from_lambda = 1;
+    TRY(res_launch(r, D.acc, 1, p, st));
+    LK(launch_stack(s->d_G.as<double>(), D.ny, D.nx_model, s->wdev[wi]->stack.p, (int)w.size(),
+                    D.grad_form, st));
+    return FWI_OK;
+}
+
 // Issue one wave's work: forward (+ misfit) and, for step 1, adjoint + stack.
 int issue_wave(fwi_survey* s, size_t wi, int step, cudaStream_t st, cudaStream_t st2) {
     const auto& D = s->desc;
     const auto& w = s->waves[wi];
+    if (s->resident) return issue_resident(s, wi, step, st);
     auto& wd = *s->wdev[wi];
     for (size_t k = 0; k < w.size(); ++k) {
         const int sh = w[k];
@@ -1794,24 +2004,7 @@ int issue_wave(fwi_survey* s, size_t wi, int step, cudaStream_t st, cudaStream_t
         const int sh = w[k];
         LK(launch_rec_last(s->d_synth.as<float>() + (size_t)s->tr_off[sh] * D.nt, D.nt, (int)s->geoms[sh].nxR.size(), st));
     }
-    // misfit + adjoint source for this wave's traces (one launch per shot:
-    // the shots of a wave need not be consecutive); the observed data may
-    // still be on their way (the batch call uploads them beside the forward
-    // pass and records obs_ready before it launches a wave); a captured wave
-    // waits for that event inside its graph
-    {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        CK(cudaStreamIsCapturing(st, &cs));
-        if (cs == cudaStreamCaptureStatusActive) CK(cudaStreamWaitEvent(st, s->obs_ready, cudaEventWaitExternal));
-        else if (s->obs_pending) CK(cudaStreamWaitEvent(st, s->obs_ready, 0));
-    }
-    for (int sh : w) {
-        const int t0 = s->tr_off[sh], t1 = s->tr_off[sh + 1];
-        if (t1 == t0) continue;
-        LK(launch_misfit(s->d_synth.as<float>() + (size_t)t0 * D.nt, s->d_obs.as<float>() + (size_t)t0 * D.nt,
-                         s->d_adj.as<float>() + (size_t)t0 * D.nt, s->d_mis_tr.as<double>() + t0, D.nt, D.dt,
-                         s->d_tr_off.as<int>(), t1 - t0, 0, nullptr, st));
-    }
+    TRY(issue_misfit(s, wi, st));
     if (step != 1) return FWI_OK;
     for (size_t k = 0; k < w.size(); ++k) {
         ShotState& ss = *s->slots[k];
@@ -1849,11 +2042,128 @@ int issue_wave(fwi_survey* s, size_t wi, int step, cudaStream_t st, cudaStream_t
 
 }  // namespace
 
+// Resident or streaming: the mean step of a gradient.  Measured, streaming
+// (all shots of a wave together) against resident: 4.1 / 2.0 us for 3 shots of
+// 40 x 90, 4.8 / 2.4 for one of 200 x 400, 9.9 / 4.7 for 12 of 163 x 384, 15 /
+// 10 for 10 of 251 x 1013, 41 / 39 for 8 windows of 600 x 1200-4000, 157 / 156
+// for 64 of 400 x 2000 (forward alone, 24 windows of 600 x 850: 49 / 34).  The
+// line: RES_GRADIENT (snapshots and imaging) times the planner's model of a
+// plain step against a fit of the streaming times.
+constexpr double RES_GRADIENT = 1.2, STREAM_STEP_US = 6.0, STREAM_CELL_US = 2.8e-6;
+
+// Resident waves of a survey: the shots' state in shared memory, a few shots
+// per launch (res_group), so that a wave needs HBM only for its snapshots and
+// accumulators.  Used unless the descriptor asks for a form of the streaming
+// kernels, keeps 16-bit snapshots, or a shot does not fit the SMs or the
+// budget.  *ok: whether the survey is resident.
+int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
+    const auto& D = s->desc;
+    *ok = false;
+    if ((D.flags & ~FWI_SURVEY_GRAPH) || D.snap_form != FWI_SNAP_F32 || D.band_rows > 0 || D.tile_kernel > 0 ||
+        D.tile_rows > 0 || D.tile_edge_rows > 0)
+        return FWI_OK;
+    size_t per = 0;
+    for (auto& l : s->lays)
+        per = std::max(per, (size_t)(s->nt_store + 1) * l.ny * l.pitch * 4 + ShotState::image_bytes(l, D.grad_form));
+    size_t most = std::min<size_t>((size_t)D.nshots, budget / std::max<size_t>(per, 1));
+    if (D.wave_shots > 0) most = std::min<size_t>(most, (size_t)D.wave_shots);
+    if (most < 1) return FWI_OK;
+    cudaStream_t st = stream();
+    if (!s->resident || (size_t)s->wave > most) {  // the plan does not depend on the time axis
+        std::vector<int> order(D.nshots);
+        for (int i = 0; i < D.nshots; ++i) order[i] = i;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return s->geoms[a].nx > s->geoms[b].nx; });
+        std::vector<const Layout*> lays;
+        for (int i : order) lays.push_back(&s->lays[i]);
+        double us = 0.0, cells = 0.0;
+        int g = res_group(lays, L().res_dev, (int)most, &us);
+        for (auto& l : s->lays) cells += (double)(l.ny + l.dn) * l.nxt;
+        if (g < 1 || RES_GRADIENT * us > STREAM_STEP_US + STREAM_CELL_US * cells) return FWI_OK;
+        const int nw = (D.nshots + g - 1) / g;
+        g = (D.nshots + nw - 1) / nw;
+        s->waves.clear();
+        s->res.clear();
+        size_t out = 0, c2 = 0;
+        for (int i = 0; i < D.nshots; i += g) {
+            s->waves.emplace_back(order.begin() + i, order.begin() + std::min(D.nshots, i + g));
+            std::vector<const ShotGeom*> geo;
+            std::vector<const Layout*> lay;
+            for (int sh : s->waves.back()) {
+                geo.push_back(&s->geoms[sh]);
+                lay.push_back(&s->lays[sh]);
+            }
+            std::unique_ptr<ResDev> r(new ResDev());
+            ResCuts cuts;
+            bool fits = res_cuts(lay, L().res_dev, cuts) && res_plan(geo, lay, cuts, L().res_dev, r->plan);
+            if (fits) TRY(res_fits(r->plan, D.acc, &fits));
+            if (!fits) {
+                s->waves.clear();
+                s->res.clear();
+                return FWI_OK;
+            }
+            TRY(res_upload(*r, st));
+            out = std::max(out, r->plan.out_elems);
+            c2 = std::max(c2, r->plan.c2_elems);
+            s->res.push_back(std::move(r));
+        }
+        s->wave = g;
+        TRY(s->res_out.ensure(std::max<size_t>(out * sizeof(uint2), 16)));
+        TRY(s->res_c2.ensure(c2 * sizeof(float)));
+    }
+    if ((int)s->slots.size() > s->wave) s->slots.resize(s->wave);
+    while ((int)s->slots.size() < s->wave) s->slots.emplace_back(new ShotState());
+    for (size_t wi = 0; wi < s->waves.size(); ++wi)
+        for (size_t k = 0; k < s->waves[wi].size(); ++k)
+            TRY(s->slots[k]->alloc_images(s->lays[s->waves[wi][k]], s->nt_store + 1, D.grad_form));
+    survey_drop_waves(s);
+    std::vector<size_t> soff(D.nshots + 1, 0);
+    for (int q = 0; q < D.nshots; ++q) soff[q + 1] = soff[q] + s->geoms[q].nxS.size();
+    for (size_t wi = 0; wi < s->waves.size(); ++wi) {
+        const auto& w = s->waves[wi];
+        std::vector<ResShot> f, a;
+        std::vector<unsigned char> stk(w.size() * stack_shot_size());
+        for (size_t k = 0; k < w.size(); ++k) {
+            const int sh = w[k];
+            const Layout& l = s->lays[sh];
+            ShotState& ss = *s->slots[k];
+            ResShot v{};
+            v.model = s->d_lambda.as<float>();
+            v.ldv = D.ny;
+            v.x0 = s->geoms[sh].x0;
+            v.srcv = s->d_src.as<float>() + soff[sh] * D.nt;
+            v.rec = s->d_synth.as<float>() + (size_t)s->tr_off[sh] * D.nt;
+            v.snaps = ss.snaps.as<float>();
+            v.k32 = ss.k.as<float>();
+            v.k64 = ss.k.as<double>();
+            v.ny = l.ny;
+            v.nx = l.nx;
+            v.dn = l.dn;
+            v.off = l.off;
+            v.pitch = l.pitch;
+            f.push_back(v);
+            v.srcv = s->d_adj.as<float>() + (size_t)s->tr_off[sh] * D.nt;
+            a.push_back(v);
+            fill_stack_shot(stk.data() + k * stack_shot_size(), ss.k.as<float>(), ss.k.as<double>(), s->geoms[sh].x0,
+                            l.nx, l.off + l.dn, l.pitch, s->gw[sh]);
+        }
+        std::unique_ptr<fwi_survey::WaveDev> wd(new fwi_survey::WaveDev());
+        TRY(upload(s->res[wi]->shots[0], f, st));
+        TRY(upload(s->res[wi]->shots[1], a, st));
+        TRY(upload(wd->stack, stk, st));
+        s->wdev.push_back(std::move(wd));
+    }
+    CK(cudaStreamSynchronize(st));
+    s->resident = true;
+    s->streaming.reset();
+    *ok = true;
+    return FWI_OK;
+}
+
 // Time-axis plan of a survey: the wave size from the HBM budget (the memory
 // the survey's slots already hold counts as available), checkpointed
 // recomputation when waves would get too small, the slots (reused; their
 // buffers only grow), the band height and the work lists of every wave.
-int survey_plan(fwi_survey* s, bool tune) {
+int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
     const auto& D = s->desc;
     s->rc_C = 0;
     size_t held = 0;
@@ -1868,6 +2178,14 @@ int survey_plan(fwi_survey* s, bool tune) {
         size_t used_resident = s->d_obs.n + s->d_synth.n + s->d_adj.n + s->d_src.n + s->d_G.n + s->d_lambda.n;
         if (s->desc.hbm_budget <= used_resident) return fail(FWI_ERR_NOMEM, "HBM budget smaller than the resident data");
         budget = std::min(budget, s->desc.hbm_budget - used_resident);
+    }
+    if (!streaming) {
+        bool res = false;
+        TRY(resident_plan(s, budget, &res));
+        if (res) return FWI_OK;
+        if (s->resident) tune = true;  // a longer time axis no longer fits: the first streaming plan
+        s->resident = false;
+        s->res.clear();
     }
     int wave = (int)std::min<size_t>((size_t)D.nshots, budget / std::max<size_t>(per, 1));
     // Checkpointed recomputation keeps a forward-state checkpoint every C steps
@@ -1909,6 +2227,41 @@ int survey_plan(fwi_survey* s, bool tune) {
     if (tune) return tune_plan(s);
     if (D.band_rows > 0) s->band = D.band_rows;
     return survey_prepare_waves(s);
+}
+
+// The survey whose streaming plan and tuning answer the query entries: *s
+// itself, or, for a resident survey, a plan of the streaming kernels for the
+// same shots, made (and tuned) on the first query; its fields are freed again.
+int streaming_view(fwi_survey** sp) {
+    fwi_survey* s = *sp;
+    if (!s->resident) return FWI_OK;
+    if (!s->streaming) {
+        std::unique_ptr<fwi_survey> c(new fwi_survey());
+        c->desc = s->desc;
+        c->nt_store = s->nt_store;
+        c->geoms = s->geoms;
+        c->lays = s->lays;
+        c->gw = s->gw;
+        c->mw = s->mw;
+        c->tr_off = s->tr_off;
+        c->ntr = s->ntr;
+        c->h_fA = s->h_fA;
+        c->h_fB = s->h_fB;
+        cudaStream_t st = stream();
+        TRY(upload(c->d_fA, c->h_fA, st));
+        TRY(upload(c->d_fB, c->h_fB, st));
+        TRY(c->d_src.alloc(s->d_src.n));
+        TRY(c->d_synth.alloc(s->d_synth.n));
+        TRY(c->d_adj.alloc(16));
+        CK(cudaMemsetAsync(c->d_src.p, 0, c->d_src.n, st));
+        TRY(survey_plan(c.get(), true, true));
+        c->slots.clear();
+        c->d_src.release();
+        c->d_synth.release();
+        s->streaming = std::move(c);
+    }
+    *sp = s->streaming.get();
+    return FWI_OK;
 }
 
 extern "C" {
@@ -1964,7 +2317,7 @@ int fwi_survey_create(const fwi_survey_desc* desc, fwi_survey** out) {
     TRY(s->d_obs.alloc(std::max<size_t>(nt * s->ntr * 4, 16)));
     TRY(s->d_synth.alloc(std::max<size_t>(nt * s->ntr * 4, 16)));
     TRY(s->d_adj.alloc(std::max<size_t>(nt * s->ntr * 4, 16)));
-    TRY(s->d_mis_tr.alloc(std::max<size_t>(s->ntr * 8, 16)));
+    TRY(s->d_mis_tr.alloc((size_t)s->ntr * 8 + 8));  // and the error word of resident launches
     TRY(s->d_mis_shot.alloc(D.nshots * 8));
     TRY(upload(s->d_tr_off, s->tr_off, st));
     TRY(s->d_G.alloc((size_t)D.ny * D.nx_model * 8));
@@ -2100,6 +2453,7 @@ int fwi_survey_run(fwi_survey* s, int step, double* misfit, float* grad) {
     const auto& D = s->desc;
     cudaStream_t st = stream();
     CK(cudaMemsetAsync(s->d_G.p, 0, s->d_G.n, st));
+    CK(cudaMemsetAsync(s->d_mis_tr.as<double>() + s->ntr, 0, 8, st));
     const int gi = step == 1 ? 0 : 1;
     for (size_t wi = 0; wi < s->waves.size(); ++wi) {
         auto& wd = *s->wdev[wi];
@@ -2161,8 +2515,8 @@ int fwi_survey_run(fwi_survey* s, int step, double* misfit, float* grad) {
         s->obs_pending = false;
     }
     // per-shot misfits (FP64) in shot order
-    std::vector<double> mis_tr(s->ntr);
-    if (s->ntr) CK(cudaMemcpyAsync(mis_tr.data(), s->d_mis_tr.p, s->ntr * 8, cudaMemcpyDeviceToHost, st));
+    std::vector<double> mis_tr(s->ntr + 1);
+    CK(cudaMemcpyAsync(mis_tr.data(), s->d_mis_tr.p, (s->ntr + 1) * 8, cudaMemcpyDeviceToHost, st));
     if (grad && step == 1) {
         const size_t n = (size_t)D.ny * D.nx_model * 4;
         const bool dev = is_device_ptr(grad);
@@ -2200,6 +2554,11 @@ int fwi_survey_run(fwi_survey* s, int step, double* misfit, float* grad) {
                 wd.recheck[g2] = true;  // the next run: direct launches once more
             }
         }
+    }
+    {
+        int err = 0;
+        std::memcpy(&err, &mis_tr[s->ntr], sizeof err);
+        TRY(res_error(err));
     }
     double tot = 0.0;
     bool finite = true;
@@ -2262,14 +2621,25 @@ int fwi_survey_two_step_bytes(fwi_survey* s, double* per_step, double* tiles_per
 }
 
 int fwi_survey_tuning(fwi_survey* s, int* wave_shots, int* band_rows) {
+    std::lock_guard<std::recursive_mutex> g(L().mu);
     if (!s) return fail(FWI_ERR_STATE, "null survey");
     if (wave_shots) *wave_shots = s->wave;
+    TRY(streaming_view(&s));
     if (band_rows) *band_rows = s->band;
     return FWI_OK;
 }
 
+int fwi_survey_resident(fwi_survey* s, int* shots_per_launch) {
+    std::lock_guard<std::recursive_mutex> g(L().mu);
+    if (!s || !shots_per_launch) return fail(FWI_ERR_STATE, "null argument");
+    *shots_per_launch = s->resident ? s->wave : 0;
+    return FWI_OK;
+}
+
 int fwi_survey_tiles(fwi_survey* s, int* tile_kernel, int* tile_rows, int* cand, float* times, int* ncand) {
+    std::lock_guard<std::recursive_mutex> g(L().mu);
     if (!s || s->wdev.empty()) return fail(FWI_ERR_STATE, "survey not prepared");
+    TRY(streaming_view(&s));
     const bool two = s->wdev[0]->n_ff > 0;
     if (tile_kernel) *tile_kernel = two ? s->tile_var + 1 : 0;
     if (tile_rows) *tile_rows = two ? s->tile_band : 0;
@@ -2284,7 +2654,9 @@ int fwi_survey_tiles(fwi_survey* s, int* tile_kernel, int* tile_rows, int* cand,
 }
 
 int fwi_survey_edge_tiles(fwi_survey* s, int* edge_rows, int* cand, float* times, int* ncand) {
+    std::lock_guard<std::recursive_mutex> g(L().mu);
     if (!s || s->wdev.empty()) return fail(FWI_ERR_STATE, "survey not prepared");
+    TRY(streaming_view(&s));
     if (edge_rows) *edge_rows = s->wdev[0]->n_ff > 0 ? s->tile_eband : 0;
     if (ncand) *ncand = NEB;
     for (int c = 0; c < NEB; ++c) {
@@ -2297,6 +2669,7 @@ int fwi_survey_edge_tiles(fwi_survey* s, int* edge_rows, int* cand, float* times
 int fwi_survey_stepping(fwi_survey* s, int* form, float* two_step_ms, float* single_ms, float* fused_ms) {
     std::lock_guard<std::recursive_mutex> g(L().mu);
     if (!s || s->wdev.empty()) return fail(FWI_ERR_STATE, "survey not prepared");
+    TRY(streaming_view(&s));
     if (form) *form = s->wdev[0]->n_ff > 0 ? 1 : (s->fused ? 2 : 0);
     if (two_step_ms) *two_step_ms = s->tune_two_ms;
     if (single_ms) *single_ms = s->tune_single_ms;
@@ -2342,6 +2715,18 @@ namespace {
 // and single steps for the rest; single_only: single steps only.
 int time_wave0_steps(fwi_survey* s, int steps, float* ms, bool single_only) {
     const auto& D = s->desc;
+    if (s->resident) {  // launches of at most nt-1 steps, each from a state at rest
+        for (int n; steps > 0; steps -= n) {
+            n = std::min(steps, D.nt - 1);
+            ResParams p = res_params(*s->res[0], 0, D.acc, D.dt, D.d, D.nt, D.store_snap, s->nt_store, D.grad_form,
+                                     s->d_fA, s->d_fB, s->res_out, s->res_c2,
+                                     reinterpret_cast<int*>(s->d_mis_tr.as<double>() + s->ntr));
+            p.from_lambda = 1;
+            p.steps = n + 1;
+            TRY(res_launch(*s->res[0], D.acc, 0, p, stream()));
+        }
+        return FWI_OK;
+    }
     auto& wd = *s->wdev[0];
     StepSet ps;
     ps.pm = base_params(D.acc, D.dt, D.store_snap, D.snap_form, D.grad_form, s->d_fA.as<float>(), s->d_fB.as<float>());

@@ -1,0 +1,672 @@
+// The resident kernel: the whole time loop of a few shots in one launch, with
+// their state in shared memory.
+//
+// A time step streams 16-20 bytes per cell through HBM when the state lives
+// there, and its kernels start and end once per step.  Here a shot's grid is
+// cut into tiles (fwi_resident.h), one thread block each; a block keeps its
+// tile's two pressure levels and CPML memory variables in shared memory from
+// the first step to the last, so a step touches global memory only for the
+// tile edges, c2 (which stays in L2), the sources, the receivers and -- every
+// store_snap steps -- the snapshots and the imaging accumulator.
+//
+// Tile edges travel as (value, step) pairs in 8-byte words: a block stores
+// the R rows and four columns along each common edge into its outbox once it
+// has computed them, and the neighbour polls the word until it carries the step
+// it waits for, so that no fence and no separate flag stand between the two.
+// Outboxes are double-buffered by step parity: a block overwrites the words
+// of step k with those of step k+2 only after its neighbours have sent step
+// k+1, which they do after they have read step k.  All blocks of a launch are
+// resident together (cooperative launch); every wait has an iteration limit,
+// after which the block sets *err and the launch ends.
+//
+// A step computes the cells its neighbours read first and sends them, then the
+// rest while they travel.  It has two barriers: after the halo of level k-1
+// has been stored (every cell of level k-1 is complete then), and before the
+// edges of level k are read for sending.
+//
+// The arithmetic is that of fwi_step.cu, expression by expression (rounded
+// multiplies and adds in the reference's order, no contraction): results are
+// bit-identical to the streaming kernels and to the reference arithmetic.
+#include "fwi_div.cuh"
+#include "fwi_resident.cuh"
+#include "fwi_stencil.cuh"
+
+namespace fwi {
+
+namespace {
+
+constexpr int RES_ROWS = 3;  // rows of interior quads computed together
+constexpr int RES_WORDS = 3;  // pairs of edge words a thread polls at a time
+constexpr int SPIN_LIMIT = 1 << 22;  // polls of one word: seconds, where a neighbour is at most microseconds behind
+
+// Edge words.  The statements name no memory: nothing else of the launch is
+// ordered against them but through the words themselves and the step's
+// barriers.
+__device__ __forceinline__ void put2(uint2* dst, float2 v, unsigned tag) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(dst), "r"(__float_as_uint(v.x)), "r"(tag),
+                 "r"(__float_as_uint(v.y)));
+}
+__device__ __forceinline__ uint4 get2(const uint2* src) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(src));
+    return v;
+}
+
+// A thread's work in one phase, packed: its quad's first column or its column
+// (16 bits), its kind + 1 (3 bits; 0: none), its rows [ya, yb) (16 bits each).
+struct ResWork {
+    unsigned xk, rows, smask;
+};
+struct ResThread {
+    const ResTile* t;      // in shared memory
+    float* sm;             // the block's shared memory
+    int kind, x, ya, yb;   // its quad's first column or its column; its rows
+    unsigned smask;        // bit r: row ya + r has a source line
+};
+
+// c2 of the tile's quads: in shared memory, or in global memory (L2) where the
+// pressure levels need the room.
+__device__ __forceinline__ const float* tile_c2(const ResParams& P, const ResThread& h) {
+    return h.t->o_c2 >= 0 ? h.sm + h.t->o_c2 : P.c2g + h.t->c2;
+}
+
+// U rows (from row y) of a thread's interior quad, no branch between the rows,
+// so that their loads and their FP32 chains overlap.  SRC: rows may have a
+// source line.  c4: c2 of the U rows.  p3, pm: new and replaced values.
+template <int R, int MODE, int U, bool SRC>
+__device__ __forceinline__ void quad_rows(const ResParams& P, const ResThread& h, const float* pc, float* pn,
+                                          const float4* c4, int y, int par, float4* p3, float4* pm) {
+    const ResTile& t = *h.t;
+    const int pitch = t.pitch;
+    float2 cp[R + 1];
+#pragma unroll
+    for (int i = 0; i <= R; ++i) cp[i] = make_float2(P.c2[i], P.c2[i]);
+    float4 q[2 * R + U];
+#pragma unroll
+    for (int i = 0; i < 2 * R + U; ++i) q[i] = ld4(pc + (i - R) * pitch);
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const float4 L = ld4(pc + j * pitch - 4), Rt = ld4(pc + j * pitch + 4);
+        pm[j] = ld4(pn + j * pitch);
+        float sv[4] = {0.f, 0.f, 0.f, 0.f};
+        if (SRC && ((h.smask >> (y + j - h.ya)) & 1u)) {
+            const int line = reinterpret_cast<const int*>(h.sm + t.o_row)[y + j - t.y0];
+            to_arr(ld4(h.sm + t.o_line + (par * t.lines[MODE] + line) * t.cp + h.x - t.x0), sv);
+        }
+        float r[4];
+        interior_update2f<R, SRC>([&](int i) { return q[j + i]; }, L, Rt, pm[j], c4[j], sv, cp, r);
+        p3[j] = from_arr(r);
+        st4(pn + j * pitch, p3[j]);
+    }
+}
+
+// Interior quads of the model rows, RES_ROWS at a time; c4: c2 of the thread's
+// first rows, loaded before a barrier.  Each block of rows reads its 2R+U rows
+// of p again: with the queue of 2R rows kept in registers between blocks (2.5
+// -> 1 shared loads of p a row, 3 moves a row) the step of three 400 x 2000
+// shots took 7.2 instead of 6.3 us.
+template <int R, int MODE>
+__device__ __forceinline__ void quads_interior(const ResParams& P, const ResThread& h, const float* cur, float* nxt,
+                                               float4 (&c4)[RES_ROWS], int par) {
+    constexpr int U = RES_ROWS;
+    const ResTile& t = *h.t;
+    const int pitch = t.pitch, cp_ = t.cp, o = (h.ya - t.y0 + R) * pitch + h.x - t.x0 + 4;
+    const float* pc = cur + o;
+    float* pn = nxt + o;
+    const float* cc = tile_c2(P, h) + (h.ya - t.y0) * cp_ + h.x - t.x0;
+    float4 p3[U], pm[U];
+    for (int y = h.ya; y < h.yb; y += U) {
+        float4 cn[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (y + U + j < h.yb) cn[j] = ld4(cc + (U + j) * cp_);
+        const int n = h.yb - y;
+        if (n >= U && ((h.smask >> (y - h.ya)) & ((1u << U) - 1u)) == 0) {
+            quad_rows<R, MODE, U, false>(P, h, pc, pn, c4, y, par, p3, pm);
+        } else {  // a shorter last block, or one with a source line: row by row
+#pragma unroll 1
+            for (int j = 0; j < U && j < n; ++j) {
+                float4 c = c4[0];
+#pragma unroll
+                for (int i = 1; i < U; ++i)
+                    if (j == i) c = c4[i];
+                quad_rows<R, MODE, 1, true>(P, h, pc + j * pitch, pn + j * pitch, &c, y + j, par, p3, pm);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) c4[j] = cn[j];
+        pc += U * pitch;
+        pn += U * pitch;
+        cc += U * cp_;
+    }
+}
+
+// The same rows one at a time on the steps that store a snapshot (MODE 0) or
+// image (MODE 1: the next row's snapshot and accumulator values are fetched
+// while a row is computed; blocks of two or three rows, their values loaded
+// together, and an L2 prefetch a step ahead were not faster).
+template <int R, int MODE>
+__device__ __forceinline__ void quads_snapshot(const ResParams& P, const ResShot& S, const ResThread& h,
+                                               const float* cur, float* nxt, int par, int snap) {
+    constexpr bool IMG = MODE == 1;
+    const ResTile& t = *h.t;
+    const int pitch = t.pitch, o = (h.ya - t.y0 + R) * pitch + h.x - t.x0 + 4;
+    const float* pc = cur + o;
+    float* pn = nxt + o;
+    const float* cc = tile_c2(P, h) + (h.ya - t.y0) * t.cp + h.x - t.x0;
+    const size_t g0 = (size_t)h.ya * S.pitch + S.off + h.x;
+    float* F = S.snaps + (size_t)snap * S.ny * S.pitch + g0;
+    double* K = P.grad_form ? S.k64 + g0 : reinterpret_cast<double*>(S.k32 + g0);
+    const size_t kp = P.grad_form ? S.pitch : S.pitch / 2;
+    float4 c, f;
+    double2 ka, kb;
+    auto fetch = [&](int r, float4& cv, float4& fv, double2& a, double2& b) {
+        cv = ld4(cc + r * t.cp);
+        if (!IMG) return;
+        fv = ldg4(F + (size_t)r * S.pitch);
+        a = *reinterpret_cast<const double2*>(K + r * kp);  // FP32 form: the row's four values
+        if (P.grad_form) b = *reinterpret_cast<const double2*>(K + r * kp + 2);
+    };
+    if (h.ya < h.yb) fetch(0, c, f, ka, kb);
+#pragma unroll 1
+    for (int y = h.ya, r = 0; y < h.yb; ++y, ++r) {
+        float4 cn = c, fn = f;
+        double2 kan = ka, kbn = kb;
+        if (y + 1 < h.yb) fetch(r + 1, cn, fn, kan, kbn);
+        float4 p3v, pmv;
+        quad_rows<R, MODE, 1, true>(P, h, pc, pn, &c, y, par, &p3v, &pmv);
+        float p3[4], pm1[4];
+        to_arr(p3v, p3);
+        to_arr(pmv, pm1);
+        if (MODE == 0) {
+            // Fields = (p_3 - p_1)*0.5/dt  (solver_acoustic_SS.f90:447)
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = div_by_const((p3[e] - pm1[e]) * 0.5f, P.dt, P.rdt);
+            st4(F + (size_t)r * S.pitch, from_arr(v));
+        } else {
+            // kernel += -0.5*(p_3-p_1)*Fields*store_snap  (:465-466)
+            float fv[4], k2[4];
+            to_arr(f, fv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) k2[e] = -(((0.5f * (p3[e] - pm1[e])) * fv[e]) * P.ss);
+            if (P.grad_form == 0) {
+                float4 kv;
+                kv.x = __int_as_float(__double2loint(ka.x)) + k2[0];
+                kv.y = __int_as_float(__double2hiint(ka.x)) + k2[1];
+                kv.z = __int_as_float(__double2loint(ka.y)) + k2[2];
+                kv.w = __int_as_float(__double2hiint(ka.y)) + k2[3];
+                *reinterpret_cast<float4*>(K + r * kp) = kv;
+            } else {
+                ka.x += (double)k2[0];
+                ka.y += (double)k2[1];
+                kb.x += (double)k2[2];
+                kb.y += (double)k2[3];
+                *reinterpret_cast<double2*>(K + r * kp) = ka;
+                *reinterpret_cast<double2*>(K + r * kp + 2) = kb;
+            }
+        }
+        c = cn;
+        f = fn;
+        ka = kan;
+        kb = kbn;
+        pc += pitch;
+        pn += pitch;
+    }
+}
+
+// Quads of the bottom pad rows: the bottom CPML strip (pml_matrices_y,
+// solver_PML_matrices.f90:42-81).  The derivatives of the clamped rows are
+// evaluated at the row they copy: p rows below nyt-1-R at row nyt-1-R, phi
+// rows outside [R, dn-1-R] of the strip at its nearest end
+// (solver_space_derivs.f90:38-53, :109-128).
+template <int R>
+__device__ __forceinline__ void quads_bottom(const ResParams& P, const ResShot& S, const ResThread& h,
+                                             const float* cur, float* nxt, int k) {
+    const ResTile& t = *h.t;
+    const int pitch = t.pitch, cp_ = t.cp, dn = S.dn, ny = S.ny, last = ny + dn - 1 - R, par = k & 1;
+    const int xo = h.x - t.x0;
+    const float* phy = h.sm + t.o_y + (par ? dn * cp_ : 0) + xo;  // old y-phi, then the new one's place
+    float* phn = h.sm + t.o_y + (par ? 0 : dn * cp_) + xo;
+    float* chy = h.sm + t.o_y + 2 * dn * cp_ + xo;
+    const float* fac = h.sm + t.o_fac;
+    float2 c1p[R + 1], c2p[R + 1];
+#pragma unroll
+    for (int i = 0; i <= R; ++i) {
+        c1p[i] = make_float2(P.c1[i], P.c1[i]);
+        c2p[i] = make_float2(P.c2[i], P.c2[i]);
+    }
+#pragma unroll 1
+    for (int y = h.ya; y < h.yb; ++y) {
+        const int jl = y - ny, yc = min(y, last), jc = min(max(jl, R), dn - 1 - R);
+        const float* pc = cur + (y - t.y0 + R) * pitch + xo + 4;
+        const float* pd = cur + (yc - t.y0 + R) * pitch + xo + 4;
+        const float4 C = ld4(pc), L = ld4(pc - 4), Rt = ld4(pc + 4);
+        const float w[12] = {L.x, L.y, L.z, L.w, C.x, C.y, C.z, C.w, Rt.x, Rt.y, Rt.z, Rt.w};
+        float* pn = nxt + (y - t.y0 + R) * pitch + xo + 4;
+        const float4 PM = ld4(pn), CC = ld4(h.sm + t.o_cb + jl * cp_ + xo);
+        const float4 PHY = ld4(phy + jl * cp_), CHY = ld4(chy + jl * cp_);
+        const float2 Ap = make_float2(fac[jl], fac[jl]), Bp = make_float2(fac[dn + jl], fac[dn + jl]);
+        float2 d2y[2], dy[2], dph[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) d2y[e] = dy[e] = dph[e] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i <= R; ++i) {
+            const float4 a = ld4(pd + i * pitch), b = ld4(pd - i * pitch);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 u = pr(a, e), d = pr(b, e);
+                d2y[e] = __fadd2_rn(d2y[e], mul0(__fadd2_rn(u, d), c2p[i]));
+                if (i) dy[e] = __fadd2_rn(dy[e], mul0(__fadd2_rn(u, make_float2(-d.x, -d.y)), c1p[i]));
+            }
+        }
+#pragma unroll
+        for (int i = 1; i <= R; ++i) {
+            const float4 a = ld4(phy + (jc + i) * cp_), b = ld4(phy + (jc - i) * cp_);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 u = pr(a, e), d = pr(b, e);
+                dph[e] = __fadd2_rn(dph[e], mul0(__fadd2_rn(u, make_float2(-d.x, -d.y)), c1p[i]));
+            }
+        }
+        float phv[4], chv[4], p3[4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float2 d2x = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i <= R; ++i) {
+                const int ia = 4 + 2 * e + i, ib = 4 + 2 * e - i;
+                d2x = __fadd2_rn(d2x, mul0(c2p[i], make_float2(w[ia] + w[ib], w[ia + 1] + w[ib + 1])));
+            }
+            const float2 phyn = __fadd2_rn(mul0(Ap, pr(PHY, e)), mul0(Bp, dy[e]));
+            const float2 chyn = __fadd2_rn(mul0(Ap, pr(CHY, e)), mul0(Bp, __fadd2_rn(d2y[e], dph[e])));
+            const float2 prop = __fadd2_rn(dph[e], chyn);
+            const float2 p = pr(C, e), pm = pr(PM, e);
+            const float2 base = __fadd2_rn(make_float2(-pm.x, -pm.y), __fadd2_rn(p, p));
+            const float2 r = __fadd2_rn(base, mul0(pr(CC, e), __fadd2_rn(__fadd2_rn(d2x, d2y[e]), prop)));
+            phv[2 * e] = phyn.x;
+            phv[2 * e + 1] = phyn.y;
+            chv[2 * e] = chyn.x;
+            chv[2 * e + 1] = chyn.y;
+            p3[2 * e] = r.x;
+            p3[2 * e + 1] = r.y;
+        }
+        st4(phn + jl * cp_, from_arr(phv));
+        st4(chy + jl * cp_, from_arr(chv));
+        st4(pn, from_arr(p3));
+    }
+}
+
+// Side-strip columns, one per thread: the x-CPML strips with the grid-edge
+// clamps and the interior columns next to them (model rows), the corners and
+// the y-CPML columns next to them (bottom pad rows).  A clamped derivative is
+// evaluated at the column or row it copies.
+template <int R, int MODE, bool SNAP, bool BOT>
+__device__ __forceinline__ void strip_columns(const ResParams& P, const ResShot& S, const ResThread& h,
+                                              const float* cur, float* nxt, int k, int snap) {
+    const ResTile& t = *h.t;
+    const int pitch = t.pitch, cp_ = t.cp, dn = S.dn, ny = S.ny, nx = S.nx, nxt_ = nx + 2 * dn, par = k & 1;
+    const int H = t.y1 - t.y0, col = h.x, xo = col - t.x0;
+    const bool right = col >= dn + nx, xc = col < dn || right;  // x-CPML column
+    const int il = right ? col - dn - nx : col;                 // its index in the dn-wide strip
+    const int cfi = right ? il : dn - 1 - col;                  // its factor (solver_PML_matrices.f90:296-312)
+    const int dcx = min(max(col, R), nxt_ - 1 - R) - col;       // column the p derivatives are taken at
+    const int dci = min(max(il, R), dn - 1 - R);                // strip column the phi derivative is taken at
+    const int ic = xc ? il : R;  // an index inside the strip arrays for every lane
+    float* xb = h.sm + (right ? t.o_xr : t.o_xl);
+    const float* phx = xb + (par ? H * dn : 0);
+    float* phxn = xb + (par ? 0 : H * dn);
+    float* chx = xb + 2 * H * dn;
+    const float* phy = h.sm + t.o_y + (par ? dn * cp_ : 0) + xo;
+    float* phyn_ = h.sm + t.o_y + (par ? 0 : dn * cp_) + xo;
+    float* chy = h.sm + t.o_y + 2 * dn * cp_ + xo;
+    const float* fac = h.sm + t.o_fac;
+    const bool left = xo < t.nl;
+    const float* c2 = h.sm + (left ? t.o_cl + xo : t.o_cr + col - (t.x1 - t.nr));
+    const int c2p = left ? t.nl : t.nr;
+    const bool src = !BOT && h.smask != 0;
+    // lanes outside the x-CPML columns run the same row with phi = chi = 0
+    // derivatives of their own (not used): no branch but the source line's
+#pragma unroll 1
+    for (int y = h.ya; y < h.yb; ++y) {
+        const int row = y - t.y0, jl = y - ny;
+        const float* pc = cur + (row + R) * pitch + xo + 4;
+        const float* px = pc + dcx;
+        const float* py = BOT ? cur + (min(y, ny + dn - 1 - R) - t.y0 + R) * pitch + xo + 4 : pc;
+        float* pn = nxt + (row + R) * pitch + xo + 4;
+        const float* fx = phx + row * dn + dci;
+        float2 a2 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);  // (d2x, d2y), (dx, dy)
+        float2 ap = make_float2(0.f, 0.f);                              // derivatives of the old (x-phi, y-phi)
+        const float* fy = BOT ? phy + min(max(jl, R), dn - 1 - R) * cp_ : fx;
+#pragma unroll
+        for (int i = 0; i <= R; ++i) {
+            const float2 hi = make_float2(px[i], py[i * pitch]), lo = make_float2(px[-i], py[-i * pitch]);
+            const float2 t1 = make_float2(P.c1[i], P.c1[i]);
+            a2 = __fadd2_rn(a2, mul0(__fadd2_rn(hi, lo), make_float2(P.c2[i], P.c2[i])));
+            if (i) {
+                a1 = __fadd2_rn(a1, mul0(__fadd2_rn(hi, make_float2(-lo.x, -lo.y)), t1));
+                const float2 fh = make_float2(fx[i], BOT ? fy[i * cp_] : 0.f);
+                const float2 fl = make_float2(fx[-i], BOT ? fy[-i * cp_] : 0.f);
+                ap = __fadd2_rn(ap, mul0(__fadd2_rn(fh, make_float2(-fl.x, -fl.y)), t1));
+            }
+        }
+        const float p = pc[0], pm1 = *pn, c = c2[row * c2p];
+        const float base = (-pm1) + 2.f * p, d2 = a2.x + a2.y;
+        // corners: factor(max(i, j)) in both directions (solver_PML_coeffs.f90:240-267)
+        const int fi = BOT ? (xc ? max(jl, cfi) : jl) : (xc ? cfi : 0);
+        const float A = fac[fi], B = fac[dn + fi];
+        const float phn = A * phx[row * dn + ic] + B * a1.x;
+        const float chn = A * chx[row * dn + ic] + B * (a2.x + ap.x);
+        const float propx = ap.x + chn;
+        float p3;
+        if (!BOT) {
+            float sv = 0.f;
+            if (src && ((h.smask >> (y - h.ya)) & 1u))
+                sv = h.sm[t.o_line + (par * t.lines[MODE] + reinterpret_cast<const int*>(h.sm + t.o_row)[row]) * cp_ + xo];
+            p3 = base + c * (d2 + (xc ? propx : sv));
+        } else {
+            const float pyn = A * phy[jl * cp_] + B * a1.y;
+            const float cyn = A * chy[jl * cp_] + B * (a2.y + ap.y);
+            const float propy = ap.y + cyn;
+            // corners in two stages (solver_acoustic_SS.f90:395-411)
+            p3 = xc ? (base + c * (d2 + propx)) + c * propy : base + c * (d2 + propy);
+            phyn_[jl * cp_] = pyn;
+            chy[jl * cp_] = cyn;
+        }
+        if (xc) {
+            phxn[row * dn + il] = phn;
+            chx[row * dn + il] = chn;
+        }
+        if (SNAP && !BOT && !xc) {
+            const size_t g = (size_t)y * S.pitch + S.off + col;
+            float* F = S.snaps + (size_t)snap * S.ny * S.pitch + g;
+            if (MODE == 0) {
+                *F = div_by_const((p3 - pm1) * 0.5f, P.dt, P.rdt);
+            } else {
+                const float k2 = -(((0.5f * (p3 - pm1)) * __ldg(F)) * P.ss);
+                if (P.grad_form == 0) S.k32[g] = S.k32[g] + k2;
+                else S.k64[g] += (double)k2;
+            }
+        }
+        *pn = p3;
+    }
+}
+
+// A pair of edge words: its first float in a pressure level's halo (bits
+// 0-15), the side (bits 16-17), whether the second word exists (bit 18).
+__device__ __forceinline__ unsigned edge_pair(int side, int dst, bool two) {
+    return (unsigned)dst | (unsigned)side << 16 | (two ? 1u << 18 : 0u);
+}
+
+template <int R, int MODE>
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResParams P) {
+    extern __shared__ float4 smem4[];
+    // per-block constants live in shared memory: the row loops need the registers
+    __shared__ ResTile tile;
+    __shared__ ResShot shot;
+    __shared__ const uint2* in[2][4];  // by parity and side: pair b of this tile is at in + 2*b
+    __shared__ uint2* own[2];          // its own outbox
+    __shared__ int o_edge[4];       // from a halo cell to the tile's own cell of the same pair
+    float* sm = reinterpret_cast<float*>(smem4);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    {
+        const int* src = reinterpret_cast<const int*>(P.tiles + blockIdx.x);
+        int* dst = reinterpret_cast<int*>(&tile);
+        for (int i = tid; i < (int)(sizeof(ResTile) / sizeof(int)); i += RES_THREADS) dst[i] = src[i];
+    }
+    __syncthreads();
+    const ResTile& t = tile;
+    if (tid == 0) {
+        shot = P.shots[t.shot];
+        for (int s = 0; s < 4; ++s) {
+            if (t.nbr[s] < 0) continue;
+            const ResTile& n = P.tiles[t.nbr[s]];
+            for (int p = 0; p < 2; ++p) in[p][s] = P.out + n.out + 2 * (p * n.npair + n.pair0[s ^ 1] - t.pair0[s]);
+        }
+        for (int p = 0; p < 2; ++p) own[p] = P.out + t.out + 2 * p * t.npair;
+        o_edge[0] = 4;
+        o_edge[1] = -4;
+        o_edge[2] = R * t.pitch;
+        o_edge[3] = -R * t.pitch;
+    }
+    __syncthreads();
+    const ResShot& S = shot;
+    const int H = t.y1 - t.y0, W = t.x1 - t.x0, dn = S.dn;
+    for (int i = tid; i < t.floats / 4; i += RES_THREADS) smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    // c2 = c**2*dt**2/d**2 with the nearest model cell in the pads
+    // (solver_acoustic_SS.f90:271-292), Vp = sqrt(lambda/1000.)
+    for (int i = tid; i < H * t.cp; i += RES_THREADS) {
+        const int x = i / H, y = i - x * H;
+        const int my = min(t.y0 + y, S.ny - 1), mx = min(max(t.x0 + x - dn, 0), S.nx - 1);
+        float v = __ldg(S.model + (size_t)my + (size_t)(S.x0 + mx) * S.ldv);
+        if (P.from_lambda) v = __fsqrt_rn(__fdiv_rn(v, 1000.f));
+        v = __fdiv_rn(__fmul_rn(__fmul_rn(v, v), P.dt2), P.d2);
+        if (t.o_c2 >= 0) sm[t.o_c2 + y * t.cp + x] = v;
+        else P.c2g[(size_t)t.c2 + y * t.cp + x] = v;
+        if (x < t.nl) sm[t.o_cl + y * t.nl + x] = v;
+        if (x < W && x >= W - t.nr) sm[t.o_cr + y * t.nr + x - (W - t.nr)] = v;
+        if (t.y0 + y >= S.ny) sm[t.o_cb + (t.y0 + y - S.ny) * t.cp + x] = v;
+    }
+    for (int i = tid; i < H; i += RES_THREADS) reinterpret_cast<int*>(sm + t.o_row)[i] = P.rows[t.rows[MODE] + i];
+    for (int i = tid; i < dn; i += RES_THREADS) {
+        sm[t.o_fac + i] = P.fA[i];
+        sm[t.o_fac + dn + i] = P.fB[i];
+    }
+    ResWork work[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        work[p] = ResWork{0, 0, 0};
+        for (int g = p ? t.ngroups[0] : 0; g < t.ngroups[0] + (p ? t.ngroups[1] : 0); ++g) {
+            const ResGroup& G = t.g[g];
+            if (warp < G.warp0 || warp >= G.warp0 + G.nwarps) continue;
+            const int i = (warp - G.warp0) * 32 + lane, b = i / G.np, c = i - b * G.np;
+            if (c >= G.n) continue;
+            const int ya = min(G.y0 + b * G.h, G.y1), yb = min(ya + G.h, G.y1);
+            work[p].xk = (unsigned)(G.x0 + (G.kind < 2 ? 4 * c : c)) | (unsigned)(G.kind + 1) << 16;
+            work[p].rows = (unsigned)ya | (unsigned)yb << 16;
+            for (int y = ya; y < yb; ++y)
+                if (P.rows[t.rows[MODE] + y - t.y0] >= 0) work[p].smask |= 1u << (y - ya);
+        }
+    }
+    auto unpack = [&](const ResWork& w) {
+        ResThread h;
+        h.t = &tile;
+        h.sm = sm;
+        h.kind = (int)(w.xk >> 16) - 1;
+        h.x = (int)(w.xk & 0xffff);
+        h.ya = (int)(w.rows & 0xffff);
+        h.yb = (int)(w.rows >> 16);
+        h.smask = w.smask;
+        return h;
+    };
+    // c2 of the first rows of a phase's interior quads, on its way while the
+    // threads poll or wait
+    float4 c4[RES_ROWS];
+    auto load_c2 = [&](const ResWork& w) {
+        const ResThread h = unpack(w);
+        if (h.kind != 0) return;
+        const float* cc = tile_c2(P, h) + (h.ya - t.y0) * t.cp + h.x - t.x0;
+#pragma unroll
+        for (int j = 0; j < RES_ROWS; ++j)
+            if (h.ya + j < h.yb) c4[j] = ld4(cc + j * t.cp);
+    };
+    // the pairs of edge words this tile reads
+    unsigned* const pairs = reinterpret_cast<unsigned*>(sm + t.o_pair);
+    const int npair = t.npair;
+    {
+        int at = 0;
+        for (int s = 0; s < 4; ++s) {
+            if (t.nbr[s] < 0) continue;
+            const int w2 = (W + 1) / 2, n = s < 2 ? 2 * H : R * w2;
+            for (int i = tid; i < n; i += RES_THREADS) {
+                if (s < 2) {
+                    const int y = i >> 1, x = 2 * (i & 1);
+                    pairs[at + i] = edge_pair(s, (R + y) * t.pitch + (s ? 4 + W : 0) + x, true);
+                } else {
+                    const int y = i / w2, x = 2 * (i - y * w2);
+                    pairs[at + i] = edge_pair(s, (s == 2 ? y : R + H + y) * t.pitch + 4 + x, x + 1 < W);
+                }
+            }
+            at += n;
+        }
+    }
+    // the tile's receivers and sources; the value of a thread's first source is fetched a step ahead
+    const int nrec = MODE == 0 && P.record ? t.rec1 - t.rec0 : 0, nsrc = t.src1[MODE] - t.src0[MODE];
+    ResRec* const recs = reinterpret_cast<ResRec*>(sm + t.o_rec);
+    ResSrc* const srcs = reinterpret_cast<ResSrc*>(sm + t.o_src);
+    for (int i = tid; i < nrec; i += RES_THREADS) recs[i] = P.rec[t.rec0 + i];
+    for (int i = tid; i < nsrc; i += RES_THREADS) srcs[i] = P.src[t.src0[MODE] + i];
+    float sval = tid < nsrc ? __ldg(S.srcv + (size_t)P.src[t.src0[MODE] + tid].vidx * P.nt) : 0.f;
+    auto record = [&](const float* p, int k) {
+        for (int e = tid; e < nrec; e += RES_THREADS) {
+            const float v = p[recs[e].off];
+            float* at = S.rec + (size_t)recs[e].ridx * P.nt;
+            at[k - 2] = v;
+            if (k == P.nt) at[P.nt - 1] = v;  // Rec_point(nt,:) = Rec_point(nt-1,:)  (solver_acoustic_SS.f90:588)
+        }
+    };
+    int l = 1, snap = MODE == 0 ? 0 : P.nt_store;
+    for (int k = 2; k <= P.steps; ++k) {
+        float* cur = sm + t.o_p[(k - 1) & 1];
+        float* nxt = sm + t.o_p[k & 1];
+        const int par = k & 1;
+        load_c2(work[0]);
+        bool ok = true;
+        if (k > 2) {
+            const unsigned tag = (unsigned)(k - 1);
+            const int pp = (k - 1) & 1;
+            for (int b = tid; b < npair && ok; b += RES_WORDS * RES_THREADS) {
+                unsigned e[RES_WORDS];
+                const uint2* src[RES_WORDS];
+                uint4 v[RES_WORDS];
+#pragma unroll
+                for (int i = 0; i < RES_WORDS; ++i) {
+                    if (b + i * RES_THREADS >= npair) continue;
+                    e[i] = pairs[b + i * RES_THREADS];
+                    src[i] = in[pp][(e[i] >> 16) & 3] + 2 * (b + i * RES_THREADS);
+                    v[i] = get2(src[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < RES_WORDS; ++i) {
+                    if (b + i * RES_THREADS >= npair) continue;
+                    const bool two = e[i] >> 18;
+                    int n = 0;
+                    while (ok && (v[i].y != tag || (two && v[i].w != tag))) {
+                        if (++n > SPIN_LIMIT || ((n & 0xfff) == 0 && *(volatile int*)P.err)) ok = false;
+                        v[i] = get2(src[i]);
+                    }
+                    *reinterpret_cast<float2*>(cur + (e[i] & 0xffff)) =
+                        make_float2(__uint_as_float(v[i].x), __uint_as_float(v[i].z));
+                }
+            }
+        }
+        // the sources of step k: S(k-1, j)
+        for (int e = tid; e < nsrc; e += RES_THREADS) {
+            const ResSrc en = srcs[e];
+            const float* at = S.srcv + (size_t)en.vidx * P.nt + (k - 2);
+            sm[t.o_line + par * t.lines[MODE] * t.cp + en.pos] = e == tid ? sval : __ldg(at);
+            if (e == tid && k < P.steps) sval = __ldg(at + 1);
+        }
+        if (__syncthreads_or(!ok)) {
+            if (tid == 0) *(volatile int*)P.err = 1;
+            return;
+        }
+        bool ev = false;
+        if (++l == P.store_snap) {
+            l = 0;
+            ev = MODE == 1 || P.store;
+            if (MODE == 0) ++snap;
+            else --snap;
+        }
+        // receivers of step k-1: every receiver gets its cell's p (:551-555)
+        if (k > 2) record(cur, k - 1);
+        // the cells the neighbours read (phase 0), then the rest
+#pragma unroll 1
+        for (int ph = 0; ph < 2; ++ph) {
+            const ResThread h = unpack(ph ? work[1] : work[0]);
+            if (h.kind == 0) {
+                if (ev) quads_snapshot<R, MODE>(P, S, h, cur, nxt, par, snap);
+                else quads_interior<R, MODE>(P, h, cur, nxt, c4, par);
+            } else if (h.kind == 1) {
+                quads_bottom<R>(P, S, h, cur, nxt, k);
+            } else if (h.kind == 2) {
+                if (ev) strip_columns<R, MODE, true, false>(P, S, h, cur, nxt, k, snap);
+                else strip_columns<R, MODE, false, false>(P, S, h, cur, nxt, k, -1);
+            } else if (h.kind == 3) {
+                strip_columns<R, MODE, false, true>(P, S, h, cur, nxt, k, snap);
+            }
+            if (ph) break;
+            load_c2(work[1]);
+            __syncthreads();
+            // The tile's edges to its neighbours: a pair's own cell lies R rows or
+            // four columns inside the halo cell that the same pair reads.  One
+            // pass of all threads over the pairs costs a barrier; storing them
+            // from the row loops, where one or two lanes of every warp hold an
+            // edge column, doubled the time of the rows.
+            if (k < P.steps)
+                for (int b = tid; b < npair; b += RES_THREADS) {
+                    const unsigned e = pairs[b];
+                    const float2 v = *reinterpret_cast<const float2*>(nxt + (e & 0xffff) + o_edge[(e >> 16) & 3]);
+                    put2(own[par] + 2 * b, v, (unsigned)k);
+                }
+        }
+    }
+    if (nrec) {
+        __syncthreads();
+        record(sm + t.o_p[P.steps & 1], P.steps);
+    }
+}
+
+using ResKernel = void (*)(const ResParams);
+
+ResKernel kernel_of(int acc, int mode) {
+    if (acc == 3) return mode == 0 ? k_resident<3, 0> : k_resident<3, 1>;
+    return mode == 0 ? k_resident<4, 0> : k_resident<4, 1>;
+}
+
+}  // namespace
+
+cudaError_t configure_resident() {
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    for (int acc = 3; acc <= 4; ++acc)
+        for (int mode = 0; mode < 2; ++mode) {
+            ResKernel k = kernel_of(acc, mode);
+            cudaFuncAttributes a;
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared);
+        }
+    return e;
+}
+
+cudaError_t resident_blocks(int acc, size_t smem, int* blocks) {
+    int a = 0, b = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel_of(acc, 0), RES_THREADS, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel_of(acc, 1), RES_THREADS, smem);
+    *blocks = a < b ? a : b;
+    return e;
+}
+
+cudaError_t launch_resident(int acc, int mode, const ResParams& p, int tiles, size_t smem, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)tiles);
+    cfg.blockDim = dim3(RES_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;  // every block resident, or the launch fails
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel_of(acc, mode), p);
+}
+
+}  // namespace fwi

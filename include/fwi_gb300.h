@@ -309,6 +309,13 @@ int fwi_survey_step_bytes(fwi_survey* s, double* bytes);
  * single-step lists their usual bytes), and the tiles' bytes of one pass.
  * Without two-step tiles per_step equals fwi_survey_step_bytes. */
 int fwi_survey_two_step_bytes(fwi_survey* s, double* per_step, double* tiles_per_pass);
+/* Resident survey: *shots_per_launch = shots whose time loop one launch runs
+ * with their state in shared memory (the first wave's; the default where it is
+ * modelled faster, the shots fit and the snapshots are FP32); 0: the survey
+ * runs the streaming kernels.  The tuning entries below describe the streaming
+ * kernels' plan for the same shots (made when first asked for): what the
+ * survey would run with one of their forms asked for in the descriptor. */
+int fwi_survey_resident(fwi_survey* s, int* shots_per_launch);
 /* Tuning chosen for the survey (wave size, band rows). */
 int fwi_survey_tuning(fwi_survey* s, int* wave_shots, int* band_rows);
 /* Two-step tiles chosen for the survey: kernel (1 = register queues, 2 =
@@ -343,7 +350,8 @@ int fwi_survey_launch_form(fwi_survey* s, int step, int* form, float* direct_ms,
  * segments (0, 0 when all snapshots are stored). */
 int fwi_survey_recompute(fwi_survey* s, int* segment_steps, int* segments);
 /* Run `steps` forward time steps of the first wave (for kernel timing; the
- * wavefields keep evolving, sources are injected). */
+ * wavefields keep evolving, sources are injected; a resident survey starts
+ * from rest). */
 int fwi_survey_time_steps(fwi_survey* s, int steps);
 
 /* calculate_misfit_gradient(iter,step,f1,f2,dt,nt,tfin,S0,Misfit,Grad) for
