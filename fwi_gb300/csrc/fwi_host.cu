@@ -713,6 +713,38 @@ Single& single() {
     return s;
 }
 
+// Device workspace of the calls that stage host arrays (misfit, beta, first
+// step, model update): buffers that only grow, kept between calls up to
+// WORK_KEPT bytes (a cudaMalloc and a cudaFree per array and call took longer
+// than the arithmetic).  The calls hold the library's lock and end with their
+// stream idle, so one set serves every thread and stream.
+struct Work {
+    static constexpr size_t WORK_KEPT = 256u << 20;
+    DBuf b[6];
+    void trim() {
+        size_t n = 0;
+        for (auto& x : b) n += x.n;
+        if (n > WORK_KEPT)
+            for (auto& x : b) x.release();
+    }
+    void release() {
+        for (auto& x : b) x.release();
+    }
+};
+Work& work() {
+    static Work w;
+    return w;
+}
+// Ends a call's use of the workspace: also after an error part-way nothing of
+// the call is in flight (on the other returns the stream is idle already).
+struct WorkCall {
+    cudaStream_t st;
+    ~WorkCall() {
+        cudaStreamSynchronize(st);
+        work().trim();
+    }
+};
+
 // The plan of fwi_misfit_gradient_batch: the survey of the last geometry seen
 // (one survey: a new geometry frees the previous one's device memory before
 // it plans, so the wave sizes always see the whole device).
@@ -829,6 +861,7 @@ int fwi_finalize(void) {
     if (!L().init) return FWI_OK;
     cudaDeviceSynchronize();
     batch_plan().release();
+    work().release();
     Single& s = single();
     s.~Single();
     new (&s) Single();
@@ -1058,13 +1091,15 @@ int fwi_misfit_function(const int* rank, const float* freq, const float* synth, 
     if (nrec < 0 || nt < 1) return fail(FWI_ERR_ARG, "NumRec must be >= 0 and nt >= 1");
     cudaStream_t st = stream();
     const size_t n = (size_t)nrec * nt;
-    DBuf ds, dob, da, dtr, doff, dms;
-    TRY(ds.alloc(n * 4));
-    TRY(dob.alloc(n * 4));
-    TRY(da.alloc(n * 4));
-    TRY(dtr.alloc(std::max(nrec, 1) * sizeof(double)));
-    TRY(doff.alloc(2 * sizeof(int)));
-    TRY(dms.alloc(sizeof(double)));
+    WorkCall wc{st};
+    DBuf &ds = work().b[0], &dob = work().b[1], &da = work().b[2], &dtr = work().b[3], &doff = work().b[4],
+         &dms = work().b[5];
+    TRY(ds.ensure(n * 4));
+    TRY(dob.ensure(n * 4));
+    TRY(da.ensure(n * 4));
+    TRY(dtr.ensure(std::max(nrec, 1) * sizeof(double)));
+    TRY(doff.ensure(2 * sizeof(int)));
+    TRY(dms.ensure(sizeof(double)));
     CK(cudaMemcpyAsync(ds.p, synth, n * 4, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dob.p, trace, n * 4, cudaMemcpyHostToDevice, st));
     const int off[2] = {0, nrec};
@@ -1089,19 +1124,20 @@ int fwi_beta_calculous(const float* Grad, const float* OldGrad, const int* nx_, 
     if (*nx_ < 1 || *ny_ < 1) return fail(FWI_ERR_ARG, "nx, ny must be >= 1");
     cudaStream_t st = stream();
     const bool dev = is_device_ptr(Grad) && is_device_ptr(OldGrad);
-    DBuf dg, dog, part, out;
+    WorkCall wc{st};
+    DBuf &dg = work().b[0], &dog = work().b[1], &part = work().b[3], &out = work().b[4];
     const float *pg = Grad, *po = OldGrad;
     if (!dev) {
-        TRY(dg.alloc(n * 4));
-        TRY(dog.alloc(n * 4));
+        TRY(dg.ensure(n * 4));
+        TRY(dog.ensure(n * 4));
         CK(cudaMemcpyAsync(dg.p, Grad, n * 4, cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(dog.p, OldGrad, n * 4, cudaMemcpyHostToDevice, st));
         pg = dg.as<float>();
         po = dog.as<float>();
     }
     const int nb = 304;
-    TRY(part.alloc(2 * nb * sizeof(double)));
-    TRY(out.alloc(2 * sizeof(double)));
+    TRY(part.ensure(2 * nb * sizeof(double)));
+    TRY(out.ensure(2 * sizeof(double)));
     LK(launch_dot(pg, po, n, part.as<double>(), nb, out.as<double>(), st));
     double h[2];
     CK(cudaMemcpyAsync(h, out.p, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -1113,19 +1149,19 @@ int fwi_beta_calculous(const float* Grad, const float* OldGrad, const int* nx_, 
 }
 
 // Inputs of the NLCG model kernels: device pointers as given, host arrays
-// staged through buffers of this call.
+// staged through the workspace.
 namespace {
 int nlcg_inputs(const float* a, const float* b, size_t n, DBuf& da, DBuf& db, const float** pa, const float** pb,
                 cudaStream_t st) {
     *pa = a;
     *pb = b;
     if (!is_device_ptr(a)) {
-        TRY(da.alloc(n * 4));
+        TRY(da.ensure(n * 4));
         CK(cudaMemcpyAsync(da.p, a, n * 4, cudaMemcpyHostToDevice, st));
         *pa = da.as<float>();
     }
     if (!is_device_ptr(b)) {
-        TRY(db.alloc(n * 4));
+        TRY(db.ensure(n * 4));
         CK(cudaMemcpyAsync(db.p, b, n * 4, cudaMemcpyHostToDevice, st));
         *pb = db.as<float>();
     }
@@ -1140,10 +1176,11 @@ int fwi_first_step(const float* Search, const float* var_orig, const int* nx_, c
     if (*nx_ < 1 || *ny_ < 1) return fail(FWI_ERR_ARG, "nx, ny must be >= 1");
     const size_t n = (size_t)(*nx_) * (*ny_);
     cudaStream_t st = stream();
-    DBuf ds, dv, dm;
+    WorkCall wc{st};
+    DBuf& dm = work().b[3];
     const float *ps = nullptr, *pv = nullptr;
-    TRY(nlcg_inputs(Search, var_orig, n, ds, dv, &ps, &pv, st));
-    TRY(dm.alloc(sizeof(unsigned)));
+    TRY(nlcg_inputs(Search, var_orig, n, work().b[0], work().b[1], &ps, &pv, st));
+    TRY(dm.ensure(sizeof(unsigned)));
     CK(cudaMemsetAsync(dm.p, 0, sizeof(unsigned), st));
     LK(launch_search_max(ps, pv, n, dm.as<unsigned>(), st));
     unsigned bits = 0;
@@ -1163,13 +1200,14 @@ int fwi_model_update(const float* Search, const float* var_orig, const float* st
     if (*nx_ < 1 || *ny_ < 1) return fail(FWI_ERR_ARG, "nx, ny must be >= 1");
     const size_t n = (size_t)(*nx_) * (*ny_);
     cudaStream_t st = stream();
-    DBuf ds, dv, dl;
+    WorkCall wc{st};
+    DBuf& dl = work().b[2];
     const float *ps = nullptr, *pv = nullptr;
-    TRY(nlcg_inputs(Search, var_orig, n, ds, dv, &ps, &pv, st));
+    TRY(nlcg_inputs(Search, var_orig, n, work().b[0], work().b[1], &ps, &pv, st));
     const bool dev_out = is_device_ptr(lambda);
     float* pl = lambda;
     if (!dev_out) {
-        TRY(dl.alloc(n * 4));
+        TRY(dl.ensure(n * 4));
         pl = dl.as<float>();
     }
     LK(launch_model_update(ps, pv, *step, n, pl, st));
