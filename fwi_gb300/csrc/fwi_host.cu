@@ -652,6 +652,7 @@ ResParams res_params(const ResDev& r, int mode, int acc, float dt, float d, int 
     p.rec = r.rec.as<ResRec>();
     p.rows = r.rows.as<int>();
     p.out = out.as<uint2>();
+    p.plane = r.plan.out_elems / 2;
     p.c2g = c2g.as<float>();
     p.err = err;
     p.fA = fA.as<float>();

@@ -9,9 +9,9 @@
 // tile edges, c2 (which stays in L2), the sources, the receivers and -- every
 // store_snap steps -- the snapshots and the imaging accumulator.
 //
-// Tile edges travel as (value, step) pairs in 8-byte words: a block stores
-// the R rows and four columns along each common edge into its outbox once it
-// has computed them, and the neighbour polls the word until it carries the step
+// Tile edges travel as (value, step) pairs in 8-byte words, each stored and
+// read whole: a block stores the R rows and four columns along each common edge
+// into its outbox, and the neighbour polls the word until it carries the step
 // it waits for, so that no fence and no separate flag stand between the two.
 // Outboxes are double-buffered by step parity: a block overwrites the words
 // of step k with those of step k+2 only after its neighbours have sent step
@@ -19,10 +19,15 @@
 // resident together (cooperative launch); every wait has an iteration limit,
 // after which the block sets *err and the launch ends.
 //
-// A step computes the cells its neighbours read first and sends them, then the
-// rest while they travel.  It has two barriers: after the halo of level k-1
-// has been stored (every cell of level k-1 is complete then), and before the
-// edges of level k are read for sending.
+// A block has twelve computing warps and four that exchange the edges, record
+// the receivers and fetch the sources.  In a step the computing warps first
+// update the cells that neighbours read (phase 0), announce that, and go on with
+// the rest (phase 1); meanwhile the others send the edges of the new level and
+// take in the neighbours' (of the new level too: its halo is read from the next
+// step on).  One barrier ends the step.  With the exchange done by the computing
+// threads -- two barriers a step, polling, sending -- a step of three 400 x
+// 2000 shots took 6.2 us instead of 5.6, one of twelve 163 x 384 shots 4.3
+// instead of 3.5, and one of 200 x 400 2.36 instead of 2.11.
 //
 // The arithmetic is that of fwi_step.cu, expression by expression (rounded
 // multiplies and adds in the reference's order, no contraction): results are
@@ -36,22 +41,43 @@ namespace fwi {
 namespace {
 
 constexpr int RES_ROWS = 3;  // rows of interior quads computed together
-constexpr int RES_WORDS = 3;  // pairs of edge words a thread polls at a time
+constexpr int RES_WORDS = 4;  // pairs of edge words a thread sends or polls at a time
 constexpr int SPIN_LIMIT = 1 << 22;  // polls of one word: seconds, where a neighbour is at most microseconds behind
 
-// Edge words.  The statements name no memory: nothing else of the launch is
-// ordered against them but through the words themselves and the step's
-// barriers.
+// Edge words, one 64-bit access each.  The statements name no memory: nothing
+// else of the launch is ordered against them but through the words themselves
+// and the step's barriers.
+__device__ __forceinline__ unsigned long long edge_word(float v, unsigned tag) {
+    return (unsigned long long)tag << 32 | __float_as_uint(v);
+}
 __device__ __forceinline__ void put2(uint2* dst, float2 v, unsigned tag) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(dst), "r"(__float_as_uint(v.x)), "r"(tag),
-                 "r"(__float_as_uint(v.y)));
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(dst), "l"(edge_word(v.x, tag)),
+                 "l"(edge_word(v.y, tag)));
 }
 __device__ __forceinline__ uint4 get2(const uint2* src) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(src));
-    return v;
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(src));
+    return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
+}
+
+// The block's barriers: all threads at the end of a step (true if any thread
+// brought `bad`), and the first phase's end, which the computing threads only
+// announce.
+__device__ __forceinline__ bool step_done(bool bad) {
+    unsigned r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 0, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((unsigned)bad)
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void edges_done() {
+    asm volatile("barrier.cta.arrive 1, %0;" ::"n"(RES_BLOCK) : "memory");
+}
+__device__ __forceinline__ void edges_wait() {
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(RES_BLOCK) : "memory");
 }
 
 // A thread's work in one phase, packed: its quad's first column or its column
@@ -401,20 +427,18 @@ __device__ __forceinline__ unsigned edge_pair(int side, int dst, bool two) {
 }
 
 template <int R, int MODE>
-__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_constant__ ResParams P) {
+__global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant__ ResParams P) {
     extern __shared__ float4 smem4[];
     // per-block constants live in shared memory: the row loops need the registers
     __shared__ ResTile tile;
     __shared__ ResShot shot;
-    __shared__ const uint2* in[2][4];  // by parity and side: pair b of this tile is at in + 2*b
-    __shared__ uint2* own[2];          // its own outbox
-    __shared__ int o_edge[4];       // from a halo cell to the tile's own cell of the same pair
+    __shared__ int in[4];           // by side: pair b of this tile is word in + 2*b of its parity's plane
     float* sm = reinterpret_cast<float*>(smem4);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     {
         const int* src = reinterpret_cast<const int*>(P.tiles + blockIdx.x);
         int* dst = reinterpret_cast<int*>(&tile);
-        for (int i = tid; i < (int)(sizeof(ResTile) / sizeof(int)); i += RES_THREADS) dst[i] = src[i];
+        for (int i = tid; i < (int)(sizeof(ResTile) / sizeof(int)); i += RES_BLOCK) dst[i] = src[i];
     }
     __syncthreads();
     const ResTile& t = tile;
@@ -423,22 +447,17 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         for (int s = 0; s < 4; ++s) {
             if (t.nbr[s] < 0) continue;
             const ResTile& n = P.tiles[t.nbr[s]];
-            for (int p = 0; p < 2; ++p) in[p][s] = P.out + n.out + 2 * (p * n.npair + n.pair0[s ^ 1] - t.pair0[s]);
+            in[s] = n.out / 2 + 2 * (n.pair0[s ^ 1] - t.pair0[s]);
         }
-        for (int p = 0; p < 2; ++p) own[p] = P.out + t.out + 2 * p * t.npair;
-        o_edge[0] = 4;
-        o_edge[1] = -4;
-        o_edge[2] = R * t.pitch;
-        o_edge[3] = -R * t.pitch;
     }
     __syncthreads();
     const ResShot& S = shot;
     const int H = t.y1 - t.y0, W = t.x1 - t.x0, dn = S.dn;
-    for (int i = tid; i < t.floats / 4; i += RES_THREADS) smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < t.floats / 4; i += RES_BLOCK) smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     // c2 = c**2*dt**2/d**2 with the nearest model cell in the pads
     // (solver_acoustic_SS.f90:271-292), Vp = sqrt(lambda/1000.)
-    for (int i = tid; i < H * t.cp; i += RES_THREADS) {
+    for (int i = tid; i < H * t.cp; i += RES_BLOCK) {
         const int x = i / H, y = i - x * H;
         const int my = min(t.y0 + y, S.ny - 1), mx = min(max(t.x0 + x - dn, 0), S.nx - 1);
         float v = __ldg(S.model + (size_t)my + (size_t)(S.x0 + mx) * S.ldv);
@@ -450,8 +469,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         if (x < W && x >= W - t.nr) sm[t.o_cr + y * t.nr + x - (W - t.nr)] = v;
         if (t.y0 + y >= S.ny) sm[t.o_cb + (t.y0 + y - S.ny) * t.cp + x] = v;
     }
-    for (int i = tid; i < H; i += RES_THREADS) reinterpret_cast<int*>(sm + t.o_row)[i] = P.rows[t.rows[MODE] + i];
-    for (int i = tid; i < dn; i += RES_THREADS) {
+    for (int i = tid; i < H; i += RES_BLOCK) reinterpret_cast<int*>(sm + t.o_row)[i] = P.rows[t.rows[MODE] + i];
+    for (int i = tid; i < dn; i += RES_BLOCK) {
         sm[t.o_fac + i] = P.fA[i];
         sm[t.o_fac + dn + i] = P.fB[i];
     }
@@ -501,7 +520,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
         for (int s = 0; s < 4; ++s) {
             if (t.nbr[s] < 0) continue;
             const int w2 = (W + 1) / 2, n = s < 2 ? 2 * H : R * w2;
-            for (int i = tid; i < n; i += RES_THREADS) {
+            for (int i = tid; i < n; i += RES_BLOCK) {
                 if (s < 2) {
                     const int y = i >> 1, x = 2 * (i & 1);
                     pairs[at + i] = edge_pair(s, (R + y) * t.pitch + (s ? 4 + W : 0) + x, true);
@@ -517,63 +536,134 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
     const int nrec = MODE == 0 && P.record ? t.rec1 - t.rec0 : 0, nsrc = t.src1[MODE] - t.src0[MODE];
     ResRec* const recs = reinterpret_cast<ResRec*>(sm + t.o_rec);
     ResSrc* const srcs = reinterpret_cast<ResSrc*>(sm + t.o_src);
-    for (int i = tid; i < nrec; i += RES_THREADS) recs[i] = P.rec[t.rec0 + i];
-    for (int i = tid; i < nsrc; i += RES_THREADS) srcs[i] = P.src[t.src0[MODE] + i];
-    float sval = tid < nsrc ? __ldg(S.srcv + (size_t)P.src[t.src0[MODE] + tid].vidx * P.nt) : 0.f;
-    auto record = [&](const float* p, int k) {
-        for (int e = tid; e < nrec; e += RES_THREADS) {
-            const float v = p[recs[e].off];
-            float* at = S.rec + (size_t)recs[e].ridx * P.nt;
-            at[k - 2] = v;
-            if (k == P.nt) at[P.nt - 1] = v;  // Rec_point(nt,:) = Rec_point(nt-1,:)  (solver_acoustic_SS.f90:588)
+    for (int i = tid; i < nrec; i += RES_BLOCK) recs[i] = P.rec[t.rec0 + i];
+    for (int i = tid; i < nsrc; i += RES_BLOCK) srcs[i] = P.src[t.src0[MODE] + i];
+    const bool comm = tid >= RES_THREADS;
+    if (comm) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RES_COMM_REGS));
+        // source values of step k, S(k-1, j), into the lines of its parity
+        const int ct = tid - RES_THREADS;
+        auto sources = [&](int k) {
+#pragma unroll 2
+            for (int e = ct; e < nsrc; e += RES_COMM) {
+                const ResSrc en = srcs[e];
+                sm[t.o_line + (k & 1) * t.lines[MODE] * t.cp + en.pos] =
+                    __ldg(S.srcv + (size_t)en.vidx * P.nt + (k - 2));
+            }
+        };
+        // receivers of level k (:551-555)
+        auto record = [&](int k) {
+            const float* p = sm + t.o_p[k & 1];
+#pragma unroll 2
+            for (int e = ct; e < nrec; e += RES_COMM) {
+                const float v = p[recs[e].off];
+                float* at = S.rec + (size_t)recs[e].ridx * P.nt;
+                at[k - 2] = v;
+                if (k == P.nt) at[P.nt - 1] = v;  // Rec_point(nt,:) = Rec_point(nt-1,:)  (solver_acoustic_SS.f90:588)
+            }
+        };
+        __syncthreads();
+        sources(2);
+        // The thread's pairs, RES_WORDS at a time: e[i] is pair b0 + i * RES_COMM
+        // (edge_pair), 0 beyond the last one.  The first ones stay in registers:
+        // shared loads take long while the others compute.
+        constexpr int STRIDE = RES_WORDS * RES_COMM;
+        unsigned kept[2][RES_WORDS];
+        auto words = [&](int b0, unsigned* e) {
+#pragma unroll
+            for (int i = 0; i < RES_WORDS; ++i) {
+                const int b = b0 + i * RES_COMM;
+                if (b0 < STRIDE) e[i] = kept[0][i];
+                else if (b0 < 2 * STRIDE) e[i] = kept[1][i];
+                else e[i] = b < npair ? pairs[b] : 0;
+            }
+        };
+        // The tile's edges to its neighbours: a pair's own cell lies R rows or
+        // four columns inside the halo cell that the same pair reads.
+        const int rows = R * t.pitch;
+        auto send = [&](const float* p, uint2* own, unsigned k, int b0, const unsigned* e) {
+            float2 v[RES_WORDS];
+#pragma unroll
+            for (int i = 0; i < RES_WORDS; ++i) {
+                const int off = e[i] >> 17 & 1 ? rows : 4;
+                if (e[i]) v[i] = *reinterpret_cast<const float2*>(p + (e[i] & 0xffff) + (e[i] >> 16 & 1 ? -off : off));
+            }
+#pragma unroll
+            for (int i = 0; i < RES_WORDS; ++i)
+                if (e[i]) put2(own + 2 * (b0 + i * RES_COMM), v[i], k);
+        };
+        // The neighbours' edges into the halo: all words that are not there yet
+        // are asked for together.
+        const int in0 = in[0], in1 = in[1], in2 = in[2], in3 = in[3];
+        auto receive = [&](float* p, const uint2* out, unsigned k, int b0, const unsigned* e) -> bool {
+            unsigned need = 0;
+            int at[RES_WORDS];
+#pragma unroll
+            for (int i = 0; i < RES_WORDS; ++i) {
+                if (e[i]) need |= 1u << i;
+                at[i] = (e[i] >> 17 & 1 ? (e[i] >> 16 & 1 ? in3 : in2) : (e[i] >> 16 & 1 ? in1 : in0)) +
+                        2 * (b0 + i * RES_COMM);
+            }
+            for (int n = 0; need; ++n) {
+                if (n > SPIN_LIMIT || ((n & 0xfff) == 0xfff && *(volatile int*)P.err)) return false;
+                uint4 v[RES_WORDS];
+#pragma unroll
+                for (int i = 0; i < RES_WORDS; ++i)
+                    if (need >> i & 1) v[i] = get2(out + at[i]);
+#pragma unroll
+                for (int i = 0; i < RES_WORDS; ++i) {
+                    if (!(need >> i & 1) || v[i].y != k || ((e[i] >> 18) && v[i].w != k)) continue;
+                    *reinterpret_cast<float2*>(p + (e[i] & 0xffff)) =
+                        make_float2(__uint_as_float(v[i].x), __uint_as_float(v[i].z));
+                    need &= ~(1u << i);
+                }
+            }
+            return true;
+        };
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2 * RES_WORDS; ++i) {
+            const int b = ct + i * RES_COMM;
+            kept[i / RES_WORDS][i % RES_WORDS] = b < npair ? pairs[b] : 0;
         }
-    };
+        for (int k = 2; k <= P.steps; ++k) {
+            float* nxt = sm + t.o_p[k & 1];
+            uint2* out = P.out + (k & 1) * P.plane;
+            uint2* own = out + t.out / 2;
+            if (k > 2) record(k - 1);
+            bool ok = true;
+            if (k < P.steps) {
+                sources(k + 1);
+                edges_wait();
+                unsigned e[RES_WORDS];
+#pragma unroll 1
+                for (int b0 = ct; b0 < npair; b0 += STRIDE) {
+                    words(b0, e);
+                    send(nxt, own, (unsigned)k, b0, e);
+                }
+#pragma unroll 1
+                for (int b0 = ct; b0 < npair && ok; b0 += STRIDE) {
+                    words(b0, e);
+                    ok = receive(nxt, out, (unsigned)k, b0, e);
+                }
+            }
+            if (step_done(!ok)) {
+                if (ct == 0) *(volatile int*)P.err = 1;
+                return;
+            }
+        }
+        record(P.steps);
+        return;
+    }
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RES_COMPUTE_REGS));
+    __syncthreads();
+    __syncthreads();
     int l = 1, snap = MODE == 0 ? 0 : P.nt_store;
     for (int k = 2; k <= P.steps; ++k) {
-        float* cur = sm + t.o_p[(k - 1) & 1];
+        const float* cur = sm + t.o_p[(k - 1) & 1];
         float* nxt = sm + t.o_p[k & 1];
         const int par = k & 1;
         load_c2(work[0]);
-        bool ok = true;
-        if (k > 2) {
-            const unsigned tag = (unsigned)(k - 1);
-            const int pp = (k - 1) & 1;
-            for (int b = tid; b < npair && ok; b += RES_WORDS * RES_THREADS) {
-                unsigned e[RES_WORDS];
-                const uint2* src[RES_WORDS];
-                uint4 v[RES_WORDS];
-#pragma unroll
-                for (int i = 0; i < RES_WORDS; ++i) {
-                    if (b + i * RES_THREADS >= npair) continue;
-                    e[i] = pairs[b + i * RES_THREADS];
-                    src[i] = in[pp][(e[i] >> 16) & 3] + 2 * (b + i * RES_THREADS);
-                    v[i] = get2(src[i]);
-                }
-#pragma unroll
-                for (int i = 0; i < RES_WORDS; ++i) {
-                    if (b + i * RES_THREADS >= npair) continue;
-                    const bool two = e[i] >> 18;
-                    int n = 0;
-                    while (ok && (v[i].y != tag || (two && v[i].w != tag))) {
-                        if (++n > SPIN_LIMIT || ((n & 0xfff) == 0 && *(volatile int*)P.err)) ok = false;
-                        v[i] = get2(src[i]);
-                    }
-                    *reinterpret_cast<float2*>(cur + (e[i] & 0xffff)) =
-                        make_float2(__uint_as_float(v[i].x), __uint_as_float(v[i].z));
-                }
-            }
-        }
-        // the sources of step k: S(k-1, j)
-        for (int e = tid; e < nsrc; e += RES_THREADS) {
-            const ResSrc en = srcs[e];
-            const float* at = S.srcv + (size_t)en.vidx * P.nt + (k - 2);
-            sm[t.o_line + par * t.lines[MODE] * t.cp + en.pos] = e == tid ? sval : __ldg(at);
-            if (e == tid && k < P.steps) sval = __ldg(at + 1);
-        }
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) *(volatile int*)P.err = 1;
-            return;
-        }
         bool ev = false;
         if (++l == P.store_snap) {
             l = 0;
@@ -581,8 +671,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
             if (MODE == 0) ++snap;
             else --snap;
         }
-        // receivers of step k-1: every receiver gets its cell's p (:551-555)
-        if (k > 2) record(cur, k - 1);
         // the cells the neighbours read (phase 0), then the rest
 #pragma unroll 1
         for (int ph = 0; ph < 2; ++ph) {
@@ -600,23 +688,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
             }
             if (ph) break;
             load_c2(work[1]);
-            __syncthreads();
-            // The tile's edges to its neighbours: a pair's own cell lies R rows or
-            // four columns inside the halo cell that the same pair reads.  One
-            // pass of all threads over the pairs costs a barrier; storing them
-            // from the row loops, where one or two lanes of every warp hold an
-            // edge column, doubled the time of the rows.
-            if (k < P.steps)
-                for (int b = tid; b < npair; b += RES_THREADS) {
-                    const unsigned e = pairs[b];
-                    const float2 v = *reinterpret_cast<const float2*>(nxt + (e & 0xffff) + o_edge[(e >> 16) & 3]);
-                    put2(own[par] + 2 * b, v, (unsigned)k);
-                }
+            if (k < P.steps) edges_done();
         }
-    }
-    if (nrec) {
-        __syncthreads();
-        record(sm + t.o_p[P.steps & 1], P.steps);
+        if (step_done(false)) return;
     }
 }
 
@@ -649,8 +723,8 @@ cudaError_t configure_resident() {
 
 cudaError_t resident_blocks(int acc, size_t smem, int* blocks) {
     int a = 0, b = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel_of(acc, 0), RES_THREADS, smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel_of(acc, 1), RES_THREADS, smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kernel_of(acc, 0), RES_BLOCK, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel_of(acc, 1), RES_BLOCK, smem);
     *blocks = a < b ? a : b;
     return e;
 }
@@ -658,7 +732,7 @@ cudaError_t resident_blocks(int acc, size_t smem, int* blocks) {
 cudaError_t launch_resident(int acc, int mode, const ResParams& p, int tiles, size_t smem, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)tiles);
-    cfg.blockDim = dim3(RES_THREADS);
+    cfg.blockDim = dim3(RES_BLOCK);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at{};

@@ -27,6 +27,7 @@ struct ResParams {
     const ResRec* rec;
     const int* rows;
     uint2* out;              // outboxes: words of a value and its step, zero before the launch
+    size_t plane;            // words of one parity: even steps, then odd steps
     float* c2g;              // c2 of all tiles, filled by the launch
     int* err;                // set when a wait for a neighbour ran out
     const float* fA;         // CPML factors (dn entries)

@@ -34,7 +34,12 @@ struct ResGroup {
 // the cells next to the tile's neighbours (the rows and columns they read),
 // then the rest while those travel.
 constexpr int RES_GROUPS = 26;
-constexpr int RES_THREADS = 384;         // threads of a block (one block per SM, up to 168 registers a thread)
+constexpr int RES_THREADS = 384;         // computing threads of a block (one block per SM),
+constexpr int RES_COMM = 128;            // threads that exchange the edges,
+constexpr int RES_BLOCK = RES_THREADS + RES_COMM;
+// and their registers: the block's 512 x 128 are dealt out again, neither side spills
+constexpr int RES_COMPUTE_REGS = 144, RES_COMM_REGS = 80;
+static_assert(RES_THREADS * RES_COMPUTE_REGS + RES_COMM * RES_COMM_REGS <= 65536, "registers of a block");
 constexpr size_t RES_STATIC_SMEM = 2048; // static shared memory of the kernel, rounded up
 
 struct ResTile {
@@ -48,9 +53,10 @@ struct ResTile {
     int lines[2];            // source lines, forward and adjoint
     int rows[2];             // first entry of the tile's row table (y1 - y0 ints), forward and adjoint
     // pairs of edge words the tile exchanges with its neighbours, the sides one after the other (each from pair0 on);
-    // its outbox holds the pairs it sends, in the same order (parity 1 follows parity 0)
+    // its outbox holds the pairs it sends, in the same order, once in the plane of the even steps and once in that of
+    // the odd ones
     int npair, pair0[4];
-    int out;                 // first word of its outbox
+    int out;                 // words of the outboxes before its own, of both planes
     int c2;                  // first element of the tile's c2 (rows of cp values) in global memory
     // shared memory (floats): pressure levels; x-CPML (left, right), y-CPML; c2 of the strip columns, of the bottom
     // pad rows and, where there is room, of the whole tile (o_c2; else -1); source lines, row table, factors, edge
