@@ -40,7 +40,7 @@ namespace fwi {
 
 namespace {
 
-constexpr int RES_ROWS = 3;  // rows of interior quads computed together
+constexpr int RES_ROWS = 3;  // rows that c2 of the interior quads is fetched ahead
 constexpr int RES_WORDS = 4;  // pairs of edge words a thread sends or polls at a time
 constexpr int SPIN_LIMIT = 1 << 22;  // polls of one word: seconds, where a neighbour is at most microseconds behind
 
@@ -98,74 +98,59 @@ __device__ __forceinline__ const float* tile_c2(const ResParams& P, const ResThr
     return h.t->o_c2 >= 0 ? h.sm + h.t->o_c2 : P.c2g + h.t->c2;
 }
 
-// U rows (from row y) of a thread's interior quad, no branch between the rows,
-// so that their loads and their FP32 chains overlap.  SRC: rows may have a
-// source line.  c4: c2 of the U rows.  p3, pm: new and replaced values.
-template <int R, int MODE, int U, bool SRC>
-__device__ __forceinline__ void quad_rows(const ResParams& P, const ResThread& h, const float* pc, float* pn,
-                                          const float4* c4, int y, int par, float4* p3, float4* pm) {
+// The source values of row y of a thread's quad.
+template <int MODE>
+__device__ __forceinline__ void source_row(const ResThread& h, int y, int par, float* sv) {
     const ResTile& t = *h.t;
-    const int pitch = t.pitch;
-    float2 cp[R + 1];
-#pragma unroll
-    for (int i = 0; i <= R; ++i) cp[i] = make_float2(P.c2[i], P.c2[i]);
-    float4 q[2 * R + U];
-#pragma unroll
-    for (int i = 0; i < 2 * R + U; ++i) q[i] = ld4(pc + (i - R) * pitch);
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-        const float4 L = ld4(pc + j * pitch - 4), Rt = ld4(pc + j * pitch + 4);
-        pm[j] = ld4(pn + j * pitch);
-        float sv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (SRC && ((h.smask >> (y + j - h.ya)) & 1u)) {
-            const int line = reinterpret_cast<const int*>(h.sm + t.o_row)[y + j - t.y0];
-            to_arr(ld4(h.sm + t.o_line + (par * t.lines[MODE] + line) * t.cp + h.x - t.x0), sv);
-        }
-        float r[4];
-        interior_update2f<R, SRC>([&](int i) { return q[j + i]; }, L, Rt, pm[j], c4[j], sv, cp, r);
-        p3[j] = from_arr(r);
-        st4(pn + j * pitch, p3[j]);
-    }
+    const int line = reinterpret_cast<const int*>(h.sm + t.o_row)[y - t.y0];
+    to_arr(ld4(h.sm + t.o_line + (par * t.lines[MODE] + line) * t.cp + h.x - t.x0), sv);
 }
 
-// Interior quads of the model rows, RES_ROWS at a time; c4: c2 of the thread's
-// first rows, loaded before a barrier.  Each block of rows reads its 2R+U rows
-// of p again: with the queue of 2R rows kept in registers between blocks (2.5
-// -> 1 shared loads of p a row, 3 moves a row) the step of three 400 x 2000
-// shots took 7.2 instead of 6.3 us.
+// Interior quads of the model rows.  The 2R+1 rows of p around the current one
+// stay in registers, row r in slot r mod 9 of an unrolled loop of nine rows, so
+// that none moves: a row takes five shared loads and a store of a quad, 24
+// wavefronts a warp beside 48 (R = 3) packed-FP32 cycles.  c2, which may come
+// from L2, is fetched three rows ahead; fetching the other values a row ahead
+// was slower (5.26 instead of 5.04 us a step of three 400 x 2000 shots), as
+// were three rows at a time with their 2R+3 rows loaded anew (5.6) and 16
+// computing warps of 104 registers (7.1: spills).
 template <int R, int MODE>
 __device__ __forceinline__ void quads_interior(const ResParams& P, const ResThread& h, const float* cur, float* nxt,
                                                float4 (&c4)[RES_ROWS], int par) {
-    constexpr int U = RES_ROWS;
+    constexpr int N = 9;
+    static_assert(2 * R + 1 <= N && N % RES_ROWS == 0, "slots");
     const ResTile& t = *h.t;
     const int pitch = t.pitch, cp_ = t.cp, o = (h.ya - t.y0 + R) * pitch + h.x - t.x0 + 4;
     const float* pc = cur + o;
     float* pn = nxt + o;
     const float* cc = tile_c2(P, h) + (h.ya - t.y0) * cp_ + h.x - t.x0;
-    float4 p3[U], pm[U];
-    for (int y = h.ya; y < h.yb; y += U) {
-        float4 cn[U];
+    int left = h.yb - h.ya;  // rows to go
+    if (left <= 0) return;
+    float2 cp[R + 1];
 #pragma unroll
-        for (int j = 0; j < U; ++j)
-            if (y + U + j < h.yb) cn[j] = ld4(cc + (U + j) * cp_);
-        const int n = h.yb - y;
-        if (n >= U && ((h.smask >> (y - h.ya)) & ((1u << U) - 1u)) == 0) {
-            quad_rows<R, MODE, U, false>(P, h, pc, pn, c4, y, par, p3, pm);
-        } else {  // a shorter last block, or one with a source line: row by row
-#pragma unroll 1
-            for (int j = 0; j < U && j < n; ++j) {
-                float4 c = c4[0];
+    for (int i = 0; i <= R; ++i) cp[i] = make_float2(P.c2[i], P.c2[i]);
+    float4 q[N];
 #pragma unroll
-                for (int i = 1; i < U; ++i)
-                    if (j == i) c = c4[i];
-                quad_rows<R, MODE, 1, true>(P, h, pc + j * pitch, pn + j * pitch, &c, y + j, par, p3, pm);
-            }
+    for (int i = 0; i <= 2 * R; ++i) q[i] = ld4(pc + (i - R) * pitch);
+    unsigned sm = h.smask;
+    while (true) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const float4 L = ld4(pc - 4), Rt = ld4(pc + 4), pm = ld4(pn);
+            float sv[4] = {0.f, 0.f, 0.f, 0.f};
+            const bool src = sm & 1u;
+            if (src) source_row<MODE>(h, h.yb - left, par, sv);
+            float r[4];
+            interior_update2f<R, true>([&](int i) { return q[(j + i) % N]; }, L, Rt, pm, c4[j % RES_ROWS], sv, cp, r, src);
+            st4(pn, from_arr(r));
+            if (left > RES_ROWS) c4[j % RES_ROWS] = ld4(cc + RES_ROWS * cp_);
+            if (--left == 0) return;
+            q[(j + 2 * R + 1) % N] = ld4(pc + (R + 1) * pitch);
+            sm >>= 1;
+            pc += pitch;
+            pn += pitch;
+            cc += cp_;
         }
-#pragma unroll
-        for (int j = 0; j < U; ++j) c4[j] = cn[j];
-        pc += U * pitch;
-        pn += U * pitch;
-        cc += U * cp_;
     }
 }
 
@@ -195,16 +180,24 @@ __device__ __forceinline__ void quads_snapshot(const ResParams& P, const ResShot
         a = *reinterpret_cast<const double2*>(K + r * kp);  // FP32 form: the row's four values
         if (P.grad_form) b = *reinterpret_cast<const double2*>(K + r * kp + 2);
     };
+    float2 cp[R + 1];
+#pragma unroll
+    for (int i = 0; i <= R; ++i) cp[i] = make_float2(P.c2[i], P.c2[i]);
     if (h.ya < h.yb) fetch(0, c, f, ka, kb);
 #pragma unroll 1
     for (int y = h.ya, r = 0; y < h.yb; ++y, ++r) {
         float4 cn = c, fn = f;
         double2 kan = ka, kbn = kb;
         if (y + 1 < h.yb) fetch(r + 1, cn, fn, kan, kbn);
-        float4 p3v, pmv;
-        quad_rows<R, MODE, 1, true>(P, h, pc, pn, &c, y, par, &p3v, &pmv);
-        float p3[4], pm1[4];
-        to_arr(p3v, p3);
+        float4 q[2 * R + 1];
+#pragma unroll
+        for (int i = 0; i <= 2 * R; ++i) q[i] = ld4(pc + (i - R) * pitch);
+        const float4 pmv = ld4(pn);
+        float p3[4], pm1[4], sv[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool src = (h.smask >> r) & 1u;
+        if (src) source_row<MODE>(h, y, par, sv);
+        interior_update2f<R, true>([&](int i) { return q[i]; }, ld4(pc - 4), ld4(pc + 4), pmv, c, sv, cp, p3, src);
+        st4(pn, from_arr(p3));
         to_arr(pmv, pm1);
         if (MODE == 0) {
             // Fields = (p_3 - p_1)*0.5/dt  (solver_acoustic_SS.f90:447)

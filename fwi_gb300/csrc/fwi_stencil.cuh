@@ -37,10 +37,10 @@ __device__ __forceinline__ float2 mul0(float2 a, float2 b) { return __ffma2_rn(a
 // reference adds it to 0, which changes nothing but the sign of a zero).
 // x-neighbour pairs at odd offsets straddle two register pairs: their sums
 // are formed with two scalar adds straight into a pair.
-// SRC: whether source values are injected (without them the reference adds 0).
+// SRC: whether source values may be injected, `src` whether they are (without them the reference adds 0).
 template <int R, bool SRC = true, typename QF>
 __device__ __forceinline__ void interior_update2f(QF q, float4 L, float4 Rt, float4 pm1, float4 cc, const float* sv,
-                                                  const float2* cp, float* p3) {
+                                                  const float2* cp, float* p3, bool src = true) {
     const float4 C = q(R);
     const float w[12] = {L.x, L.y, L.z, L.w, C.x, C.y, C.z, C.w, Rt.x, Rt.y, Rt.z, Rt.w};
 #pragma unroll
@@ -65,7 +65,7 @@ __device__ __forceinline__ void interior_update2f(QF q, float4 L, float4 Rt, flo
         const float2 pm = pr(pm1, k);
         const float2 t = __fadd2_rn(make_float2(-pm.x, -pm.y), p2);
         float2 d = __fadd2_rn(ax, ay);
-        if (SRC) d = __fadd2_rn(d, make_float2(sv[2 * k], sv[2 * k + 1]));
+        if (SRC && src) d = __fadd2_rn(d, make_float2(sv[2 * k], sv[2 * k + 1]));
         const float2 u = mul0(d, pr(cc, k));
         const float2 r = __fadd2_rn(t, u);
         p3[2 * k] = r.x;
