@@ -177,8 +177,8 @@ __device__ __forceinline__ void quads_snapshot(const ResParams& P, const ResShot
         cv = ld4(cc + r * t.cp);
         if (!IMG) return;
         fv = ldg4(F + (size_t)r * S.pitch);
-        a = *reinterpret_cast<const double2*>(K + r * kp);  // FP32 form: the row's four values
-        if (P.grad_form) b = *reinterpret_cast<const double2*>(K + r * kp + 2);
+        if (P.grad_form) ld_d4(K + r * kp, a, b);
+        else a = *reinterpret_cast<const double2*>(K + r * kp);  // FP32 form: the row's four values
     };
     float2 cp[R + 1];
 #pragma unroll
@@ -223,8 +223,7 @@ __device__ __forceinline__ void quads_snapshot(const ResParams& P, const ResShot
                 ka.y += (double)k2[1];
                 kb.x += (double)k2[2];
                 kb.y += (double)k2[3];
-                *reinterpret_cast<double2*>(K + r * kp) = ka;
-                *reinterpret_cast<double2*>(K + r * kp + 2) = kb;
+                st_d4(K + r * kp, ka, kb);
             }
         }
         c = cn;
