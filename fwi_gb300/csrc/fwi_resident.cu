@@ -418,6 +418,52 @@ __device__ __forceinline__ unsigned edge_pair(int side, int dst, bool two) {
     return (unsigned)dst | (unsigned)side << 16 | (two ? 1u << 18 : 0u);
 }
 
+// Edge words of a communicating thread: edge_pair of each (0: none), the tile's
+// own cell that it sends, the neighbour's word that it takes in.  W of them at
+// a time: as many as the tile has for a thread, for the instructions of a pass
+// are fetched anew in every step (tiny tiles with one or two: 1.66 -> 1.52 us).
+struct EdgeWords {
+    unsigned e[RES_WORDS];
+    int cell[RES_WORDS], at[RES_WORDS];
+};
+
+// The tile's edges to its neighbours.
+template <int W>
+__device__ __forceinline__ void send_words(const float* p, uint2* own, unsigned k, const EdgeWords& w) {
+    float2 v[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+        if (w.e[i]) v[i] = *reinterpret_cast<const float2*>(p + w.cell[i]);
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+        if (w.e[i]) put2(own + 2 * i * RES_COMM, v[i], k);
+}
+
+// The neighbours' edges into the halo: all words that are not there yet are
+// asked for together.  False when the wait runs out.
+template <int W>
+__device__ __forceinline__ bool receive_words(float* p, const uint2* out, unsigned k, const EdgeWords& w, int* err) {
+    unsigned need = 0;
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+        if (w.e[i]) need |= 1u << i;
+    for (int n = 0; need; ++n) {
+        if (n > SPIN_LIMIT || ((n & 0xfff) == 0xfff && *(volatile int*)err)) return false;
+        uint4 v[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            if (need >> i & 1) v[i] = get2(out + w.at[i]);
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            if (!(need >> i & 1) || v[i].y != k || ((w.e[i] >> 18) && v[i].w != k)) continue;
+            *reinterpret_cast<float2*>(p + (w.e[i] & 0xffff)) =
+                make_float2(__uint_as_float(v[i].x), __uint_as_float(v[i].z));
+            need &= ~(1u << i);
+        }
+    }
+    return true;
+}
+
 template <int R, int MODE>
 __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant__ ResParams P) {
     extern __shared__ float4 smem4[];
@@ -532,11 +578,10 @@ __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant
     for (int i = tid; i < nsrc; i += RES_BLOCK) srcs[i] = P.src[t.src0[MODE] + i];
     const bool comm = tid >= RES_THREADS;
     if (comm) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RES_COMM_REGS));
         // source values of step k, S(k-1, j), into the lines of its parity
         const int ct = tid - RES_THREADS;
         auto sources = [&](int k) {
-#pragma unroll 2
+#pragma unroll 1
             for (int e = ct; e < nsrc; e += RES_COMM) {
                 const ResSrc en = srcs[e];
                 sm[t.o_line + (k & 1) * t.lines[MODE] * t.cp + en.pos] =
@@ -546,7 +591,7 @@ __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant
         // receivers of level k (:551-555)
         auto record = [&](int k) {
             const float* p = sm + t.o_p[k & 1];
-#pragma unroll 2
+#pragma unroll 1
             for (int e = ct; e < nrec; e += RES_COMM) {
                 const float v = p[recs[e].off];
                 float* at = S.rec + (size_t)recs[e].ridx * P.nt;
@@ -556,87 +601,68 @@ __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant
         };
         __syncthreads();
         sources(2);
-        // The thread's pairs, RES_WORDS at a time: e[i] is pair b0 + i * RES_COMM
-        // (edge_pair), 0 beyond the last one.  The first ones stay in registers:
-        // shared loads take long while the others compute.
+        // The thread's pairs, RES_WORDS at a time: where the words from pair b0 on
+        // lie (e: edge_pair, 0 beyond the last one).
+        const int in0 = in[0], in1 = in[1], in2 = in[2], in3 = in[3], rows = R * t.pitch;
+        auto words = [&](EdgeWords& w, int b0, const unsigned* e) {
+#pragma unroll
+            for (int i = 0; i < RES_WORDS; ++i) {
+                // a pair's own cell lies R rows or four columns inside the halo cell that the same pair reads
+                const bool hi = e[i] >> 16 & 1, row = e[i] >> 17 & 1;
+                const int off = row ? rows : 4;
+                w.e[i] = e[i];
+                w.cell[i] = (int)(e[i] & 0xffff) + (hi ? -off : off);
+                w.at[i] = (row ? (hi ? in3 : in2) : (hi ? in1 : in0)) + 2 * (b0 + i * RES_COMM);
+            }
+        };
         constexpr int STRIDE = RES_WORDS * RES_COMM;
-        unsigned kept[2][RES_WORDS];
-        auto words = [&](int b0, unsigned* e) {
-#pragma unroll
-            for (int i = 0; i < RES_WORDS; ++i) {
-                const int b = b0 + i * RES_COMM;
-                if (b0 < STRIDE) e[i] = kept[0][i];
-                else if (b0 < 2 * STRIDE) e[i] = kept[1][i];
-                else e[i] = b < npair ? pairs[b] : 0;
-            }
-        };
-        // The tile's edges to its neighbours: a pair's own cell lies R rows or
-        // four columns inside the halo cell that the same pair reads.
-        const int rows = R * t.pitch;
-        auto send = [&](const float* p, uint2* own, unsigned k, int b0, const unsigned* e) {
-            float2 v[RES_WORDS];
-#pragma unroll
-            for (int i = 0; i < RES_WORDS; ++i) {
-                const int off = e[i] >> 17 & 1 ? rows : 4;
-                if (e[i]) v[i] = *reinterpret_cast<const float2*>(p + (e[i] & 0xffff) + (e[i] >> 16 & 1 ? -off : off));
-            }
-#pragma unroll
-            for (int i = 0; i < RES_WORDS; ++i)
-                if (e[i]) put2(own + 2 * (b0 + i * RES_COMM), v[i], k);
-        };
-        // The neighbours' edges into the halo: all words that are not there yet
-        // are asked for together.
-        const int in0 = in[0], in1 = in[1], in2 = in[2], in3 = in[3];
-        auto receive = [&](float* p, const uint2* out, unsigned k, int b0, const unsigned* e) -> bool {
-            unsigned need = 0;
-            int at[RES_WORDS];
-#pragma unroll
-            for (int i = 0; i < RES_WORDS; ++i) {
-                if (e[i]) need |= 1u << i;
-                at[i] = (e[i] >> 17 & 1 ? (e[i] >> 16 & 1 ? in3 : in2) : (e[i] >> 16 & 1 ? in1 : in0)) +
-                        2 * (b0 + i * RES_COMM);
-            }
-            for (int n = 0; need; ++n) {
-                if (n > SPIN_LIMIT || ((n & 0xfff) == 0xfff && *(volatile int*)P.err)) return false;
-                uint4 v[RES_WORDS];
-#pragma unroll
-                for (int i = 0; i < RES_WORDS; ++i)
-                    if (need >> i & 1) v[i] = get2(out + at[i]);
-#pragma unroll
-                for (int i = 0; i < RES_WORDS; ++i) {
-                    if (!(need >> i & 1) || v[i].y != k || ((e[i] >> 18) && v[i].w != k)) continue;
-                    *reinterpret_cast<float2*>(p + (e[i] & 0xffff)) =
-                        make_float2(__uint_as_float(v[i].x), __uint_as_float(v[i].z));
-                    need &= ~(1u << i);
-                }
-            }
-            return true;
-        };
         __syncthreads();
+        // those of the first passes stay in registers: shared loads take long while the others compute
+        EdgeWords first, more;
+        unsigned e[RES_WORDS], second[RES_WORDS];
+        auto load = [&](int b0, unsigned* e) {
 #pragma unroll
-        for (int i = 0; i < 2 * RES_WORDS; ++i) {
-            const int b = ct + i * RES_COMM;
-            kept[i / RES_WORDS][i % RES_WORDS] = b < npair ? pairs[b] : 0;
-        }
+            for (int i = 0; i < RES_WORDS; ++i) e[i] = b0 + i * RES_COMM < npair ? pairs[b0 + i * RES_COMM] : 0;
+        };
+        load(ct, e);
+        words(first, ct, e);
+        load(ct + STRIDE, second);
+        auto next_words = [&](int b0) {
+            if (b0 >= 2 * STRIDE) {
+                load(b0, e);
+                words(more, b0, e);
+            } else {
+                words(more, b0, second);
+            }
+        };
+        const int nwords = (npair + RES_COMM - 1) / RES_COMM;  // of a thread
         for (int k = 2; k <= P.steps; ++k) {
             float* nxt = sm + t.o_p[k & 1];
             uint2* out = P.out + (k & 1) * P.plane;
-            uint2* own = out + t.out / 2;
+            uint2* own = out + t.out / 2 + 2 * ct;
+            const unsigned tag = (unsigned)k;
             if (k > 2) record(k - 1);
             bool ok = true;
             if (k < P.steps) {
                 sources(k + 1);
                 edges_wait();
-                unsigned e[RES_WORDS];
+                if (nwords <= 1) send_words<1>(nxt, own, tag, first);
+                else if (nwords == 2) send_words<2>(nxt, own, tag, first);
+                else if (nwords == 3) send_words<3>(nxt, own, tag, first);
+                else send_words<RES_WORDS>(nxt, own, tag, first);
 #pragma unroll 1
-                for (int b0 = ct; b0 < npair; b0 += STRIDE) {
-                    words(b0, e);
-                    send(nxt, own, (unsigned)k, b0, e);
+                for (int b0 = ct + STRIDE; b0 < npair; b0 += STRIDE) {
+                    next_words(b0);
+                    send_words<RES_WORDS>(nxt, own + 2 * (b0 - ct), tag, more);
                 }
+                if (nwords <= 1) ok = receive_words<1>(nxt, out, tag, first, P.err);
+                else if (nwords == 2) ok = receive_words<2>(nxt, out, tag, first, P.err);
+                else if (nwords == 3) ok = receive_words<3>(nxt, out, tag, first, P.err);
+                else ok = receive_words<RES_WORDS>(nxt, out, tag, first, P.err);
 #pragma unroll 1
-                for (int b0 = ct; b0 < npair && ok; b0 += STRIDE) {
-                    words(b0, e);
-                    ok = receive(nxt, out, (unsigned)k, b0, e);
+                for (int b0 = ct + STRIDE; b0 < npair && ok; b0 += STRIDE) {
+                    next_words(b0);
+                    ok = receive_words<RES_WORDS>(nxt, out, tag, more, P.err);
                 }
             }
             if (step_done(!ok)) {
@@ -647,7 +673,6 @@ __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant
         record(P.steps);
         return;
     }
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RES_COMPUTE_REGS));
     __syncthreads();
     __syncthreads();
     int l = 1, snap = MODE == 0 ? 0 : P.nt_store;
@@ -679,8 +704,8 @@ __global__ void __launch_bounds__(RES_BLOCK, 1) k_resident(const __grid_constant
                 strip_columns<R, MODE, false, true>(P, S, h, cur, nxt, k, snap);
             }
             if (ph) break;
-            load_c2(work[1]);
             if (k < P.steps) edges_done();
+            load_c2(work[1]);
         }
         if (step_done(false)) return;
     }

@@ -34,12 +34,9 @@ struct ResGroup {
 // the cells next to the tile's neighbours (the rows and columns they read),
 // then the rest while those travel.
 constexpr int RES_GROUPS = 26;
-constexpr int RES_THREADS = 384;         // computing threads of a block (one block per SM),
-constexpr int RES_COMM = 128;            // threads that exchange the edges,
+constexpr int RES_THREADS = 384;         // computing threads of a block (one block per SM) and
+constexpr int RES_COMM = 128;            // threads that exchange the edges: 128 registers each (144 and 80: no faster)
 constexpr int RES_BLOCK = RES_THREADS + RES_COMM;
-// and their registers: the block's 512 x 128 are dealt out again, neither side spills
-constexpr int RES_COMPUTE_REGS = 144, RES_COMM_REGS = 80;
-static_assert(RES_THREADS * RES_COMPUTE_REGS + RES_COMM * RES_COMM_REGS <= 65536, "registers of a block");
 constexpr size_t RES_STATIC_SMEM = 2048; // static shared memory of the kernel, rounded up
 
 struct ResTile {
