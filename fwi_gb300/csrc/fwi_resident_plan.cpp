@@ -202,12 +202,16 @@ bool cut_shot(const Layout& l, int most, size_t cap, bool c2_shared, ResCut& bes
                     c.smem = std::max(c.smem, (size_t)t.floats * 4);
                     if (c.smem > cap) ok = false;
                     double us = STEP_US + PAIR_US * ((t.npair + RES_THREADS - 1) / RES_THREADS);
+                    // a tile marches no fewer rows than its quads over all threads: cuts that cannot win end here
+                    const double least = (t.y1 - t.y0) * ((t.x1 - t.x0) / 4) / (double)RES_THREADS;
+                    if (found && us + std::min(ROW_US[0], ROW_US[1]) * least >= best.us) ok = false;
                     for (int p = 0; p < 2 && ok; ++p) {
                         const double r = min_rows(l, Rect{t.x0, t.x1, t.y0, t.y1}, p);
                         if (r < 0) ok = false;
                         us += ROW_US[p] * r;
                     }
                     c.us = std::max(c.us, us);
+                    if (found && c.us >= best.us) ok = false;
                 }
             }
             if (!ok) continue;
