@@ -33,24 +33,17 @@ __device__ __forceinline__ float div_main(float a, float b, float y) {
     return __fmaf_rn(r, y, q);
 }
 
-// RN(a/b) for 0 < |a| < 2^-100.  A normal quotient is that of a*2^64 (a
-// normal dividend) scaled back by 2^-64, exactly.  A quotient below 2^-126
-// lies on the grid of multiples of 2^-149: n = the integer nearest to
-// s/b, s = a*2^149 (exact), ties to even, from c = RN(s/b) rounded to an
-// integer n0 and the exact remainder r = s - n0*b (one FMA): |r| > b/2 moves
-// n0 one step towards r, |r| = b/2 is a tie; the quotient is n*2^-149 with
-// the sign of a.
+// RN(a/b) for 0 < |a| < 2^-100: the quotient q of a*2^64 (a normal dividend)
+// scaled back by 2^-64, exactly if it is normal.  A quotient below 2^-126 is
+// rounded a second time, to a multiple t of 2^-149; that is RN(a/b) as long as
+// q is not half-way between two of them, or is the quotient itself.  Else
+// a/b lies on the side of the exact remainder: where t is on the other one,
+// the neighbour across q is the result.
 __device__ __forceinline__ float div_tiny(float a, float b, float y) {
-    const float qs = __fmul_rn(div_main(__fmul_rn(a, 0x1p64f), b, y), 0x1p-64f);
-    const float s = __fmul_rn(__fmul_rn(a, 0x1p100f), 0x1p49f);
-    const float n0 = rintf(div_main(s, b, y));
-    const float r = __fmaf_rn(-n0, b, s);
-    const float hb = __fmul_rn(0.5f, b), ar = fabsf(r);
-    const float h = __fmul_rn(n0, 0.5f);
-    const bool up = ar > hb || (ar == hb && truncf(h) != h);
-    const float n = up ? __fadd_rn(n0, copysignf(1.f, r)) : n0;
-    const float qi = copysignf(__fmul_rn(n, 0x1p-149f), a);
-    return fabsf(qs) >= 0x1p-126f ? qs : qi;
+    const float s = __fmul_rn(a, 0x1p64f), q = div_main(s, b, y), r = __fmaf_rn(-q, b, s);
+    const float t = __fmul_rn(q, 0x1p-64f), d = __fmaf_rn(t, -0x1p64f, q);
+    const bool across = fabsf(d) == 0x1p-86f && r != 0.f && (r > 0.f) == (d > 0.f);
+    return across ? __fadd_rn(t, copysignf(0x1p-149f, d)) : t;
 }
 
 __device__ __forceinline__ float div_by_const(float a, float b, float y) {
@@ -60,6 +53,37 @@ __device__ __forceinline__ float div_by_const(float a, float b, float y) {
     else if (m < 0x1p-100f && y != 0.f) q = div_tiny(a, b, y);
     else if (!(m <= 0x1p100f) || y == 0.f) q = __fdiv_rn(a, b);
     return q;
+}
+
+// Four of them in place: the quotients of all four at once, then one branch for
+// the tiny dividends and one for the other exceptions.  The precursor is tiny
+// almost everywhere, and its quotients go through the longest chain: with a
+// branch per cell and the double-rounded quotients formed from integers, a
+// snapshot step of three 400 x 2000 shots took 7.0 us more than another one,
+// now 2.8.
+__device__ __forceinline__ void div4_by_const(float* a, float b, float y) {
+    float q[4];
+    bool tiny = false, other = y == 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float m = fabsf(a[e]);
+        q[e] = m == 0.f ? a[e] : div_main(a[e], b, y);
+        tiny |= m < 0x1p-100f && m != 0.f;
+        other |= !(m <= 0x1p100f);
+    }
+    if (tiny) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float t = div_tiny(a[e], b, y), m = fabsf(a[e]);
+            if (m < 0x1p-100f && m != 0.f) q[e] = t;
+        }
+    }
+    if (other) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) q[e] = div_by_const(a[e], b, y);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) a[e] = q[e];
 }
 
 }  // namespace fwi

@@ -203,7 +203,8 @@ __device__ __forceinline__ void quads_snapshot(const ResParams& P, const ResShot
             // Fields = (p_3 - p_1)*0.5/dt  (solver_acoustic_SS.f90:447)
             float v[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = div_by_const((p3[e] - pm1[e]) * 0.5f, P.dt, P.rdt);
+            for (int e = 0; e < 4; ++e) v[e] = (p3[e] - pm1[e]) * 0.5f;
+            div4_by_const(v, P.dt, P.rdt);
             st4(F + (size_t)r * S.pitch, from_arr(v));
         } else {
             // kernel += -0.5*(p_3-p_1)*Fields*store_snap  (:465-466)
