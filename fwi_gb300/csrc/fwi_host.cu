@@ -2082,12 +2082,13 @@ int issue_wave(fwi_survey* s, size_t wi, int step, cudaStream_t st, cudaStream_t
 }  // namespace
 
 // Resident or streaming: the mean step of a gradient.  Measured, streaming
-// (all shots of a wave together) against resident: 4.1 / 2.0 us for 3 shots of
-// 40 x 90, 4.8 / 2.4 for one of 200 x 400, 9.9 / 4.7 for 12 of 163 x 384, 15 /
-// 10 for 10 of 251 x 1013, 41 / 39 for 8 windows of 600 x 1200-4000, 157 / 156
-// for 64 of 400 x 2000 (forward alone, 24 windows of 600 x 850: 49 / 34).  The
+// (all shots of a wave together) against resident: 3.9 / 1.8 us for 3 shots of
+// 40 x 90, 4.6 / 1.8 for one of 200 x 400, 9.9 / 3.5 for 12 of 163 x 384, 15 /
+// 7.9 for 10 of 251 x 1013, 42 / 30 for 8 windows of 600 x 1200-4000, 157 / 123
+// for 64 of 400 x 2000 (forward alone, 24 windows of 600 x 850: 49 / 27).  The
 // line: RES_GRADIENT (snapshots and imaging) times the planner's model of a
-// plain step against a fit of the streaming times.
+// plain step against a fit of the streaming times.  The model reads high
+// (fwi_resident_plan.cpp), so near the line the streaming kernels are kept.
 constexpr double RES_GRADIENT = 1.2, STREAM_STEP_US = 6.0, STREAM_CELL_US = 2.8e-6;
 
 // Resident waves of a survey: the shots' state in shared memory, a few shots

@@ -27,7 +27,8 @@
 // step on).  One barrier ends the step.  With the exchange done by the computing
 // threads -- two barriers a step, polling, sending -- a step of three 400 x
 // 2000 shots took 6.2 us instead of 5.6, one of twelve 163 x 384 shots 4.3
-// instead of 3.5, and one of 200 x 400 2.36 instead of 2.11.
+// instead of 3.5, and one of 200 x 400 2.36 instead of 2.11 (now 5.0, 3.2 and
+// 1.85: the row loops and the exchange have become shorter since).
 //
 // The arithmetic is that of fwi_step.cu, expression by expression (rounded
 // multiplies and adds in the reference's order, no contraction): results are
