@@ -347,12 +347,25 @@ __device__ __forceinline__ void strip_columns(const ResParams& P, const ResShot&
     const float* c2 = h.sm + (left ? t.o_cl + xo : t.o_cr + col - (t.x1 - t.nr));
     const int c2p = left ? t.nl : t.nr;
     const bool src = !BOT && h.smask != 0;
+    // the column's rows around the current one (model rows; a third of the loads
+    // of a row would be theirs)
+    float qy[2 * R + 1];
+    if (!BOT) {
+        const float* p0 = cur + (h.ya - t.y0) * pitch + xo + 4;
+#pragma unroll
+        for (int i = 0; i < 2 * R; ++i) qy[i + 1] = p0[i * pitch];
+    }
     // lanes outside the x-CPML columns run the same row with phi = chi = 0
     // derivatives of their own (not used): no branch but the source line's
 #pragma unroll 1
     for (int y = h.ya; y < h.yb; ++y) {
         const int row = y - t.y0, jl = y - ny;
         const float* pc = cur + (row + R) * pitch + xo + 4;
+        if (!BOT) {
+#pragma unroll
+            for (int i = 0; i < 2 * R; ++i) qy[i] = qy[i + 1];
+            qy[2 * R] = pc[R * pitch];
+        }
         const float* px = pc + dcx;
         const float* py = BOT ? cur + (min(y, ny + dn - 1 - R) - t.y0 + R) * pitch + xo + 4 : pc;
         float* pn = nxt + (row + R) * pitch + xo + 4;
@@ -362,7 +375,8 @@ __device__ __forceinline__ void strip_columns(const ResParams& P, const ResShot&
         const float* fy = BOT ? phy + min(max(jl, R), dn - 1 - R) * cp_ : fx;
 #pragma unroll
         for (int i = 0; i <= R; ++i) {
-            const float2 hi = make_float2(px[i], py[i * pitch]), lo = make_float2(px[-i], py[-i * pitch]);
+            const float2 hi = make_float2(px[i], BOT ? py[i * pitch] : qy[R + i]);
+            const float2 lo = make_float2(px[-i], BOT ? py[-i * pitch] : qy[R - i]);
             const float2 t1 = make_float2(P.c1[i], P.c1[i]);
             a2 = __fadd2_rn(a2, mul0(__fadd2_rn(hi, lo), make_float2(P.c2[i], P.c2[i])));
             if (i) {
@@ -372,7 +386,7 @@ __device__ __forceinline__ void strip_columns(const ResParams& P, const ResShot&
                 ap = __fadd2_rn(ap, mul0(__fadd2_rn(fh, make_float2(-fl.x, -fl.y)), t1));
             }
         }
-        const float p = pc[0], pm1 = *pn, c = c2[row * c2p];
+        const float p = BOT ? pc[0] : qy[R], pm1 = *pn, c = c2[row * c2p];
         const float base = (-pm1) + 2.f * p, d2 = a2.x + a2.y;
         // corners: factor(max(i, j)) in both directions (solver_PML_coeffs.f90:240-267)
         const int fi = BOT ? (xc ? max(jl, cfi) : jl) : (xc ? cfi : 0);
