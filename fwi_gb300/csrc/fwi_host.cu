@@ -2085,11 +2085,15 @@ int issue_wave(fwi_survey* s, size_t wi, int step, cudaStream_t st, cudaStream_t
 // (all shots of a wave together) against resident: 3.9 / 1.8 us for 3 shots of
 // 40 x 90, 4.6 / 1.8 for one of 200 x 400, 9.9 / 3.5 for 12 of 163 x 384, 15 /
 // 7.9 for 10 of 251 x 1013, 42 / 30 for 8 windows of 600 x 1200-4000, 157 / 123
-// for 64 of 400 x 2000 (forward alone, 24 windows of 600 x 850: 49 / 27).  The
-// line: RES_GRADIENT (snapshots and imaging) times the planner's model of a
-// plain step against a fit of the streaming times.  The model reads high
-// (fwi_resident_plan.cpp), so near the line the streaming kernels are kept.
-constexpr double RES_GRADIENT = 1.2, STREAM_STEP_US = 6.0, STREAM_CELL_US = 2.8e-6;
+// for 64 of 400 x 2000 (forward alone, 24 windows of 600 x 850: 49 / 27), 51 /
+// 29 for 64 of 163 x 700, 45 / 25 for 64 of 400 x 200, 69 / 34 for 64 of
+// 600 x 200, 36 / 21 for 4 of 600 x 4000.  The line: RES_GRADIENT (snapshots
+// and imaging) times the planner's model of a plain step against a fit of the
+// streaming times that stays up to 30 % below them: a step's launches, its
+// model cells, its side strips and its bottom pad.  (A line by cells alone left
+// three of the last four sizes and 30 windows of 600 x 1200-4000 streaming.)
+constexpr double RES_GRADIENT = 1.2, STREAM_STEP_US = 4.0;
+constexpr double STREAM_CELL_US = 2.0e-6, STREAM_SIDE_US = 12.0e-6, STREAM_BOTTOM_US = 8.0e-6;
 
 // Resident waves of a survey: the shots' state in shared memory, a few shots
 // per launch (res_group), so that a wave needs HBM only for its snapshots and
@@ -2115,10 +2119,11 @@ int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return s->geoms[a].nx > s->geoms[b].nx; });
         std::vector<const Layout*> lays;
         for (int i : order) lays.push_back(&s->lays[i]);
-        double us = 0.0, cells = 0.0;
+        double us = 0.0, streaming = STREAM_STEP_US;
         int g = res_group(lays, L().res_dev, (int)most, &us);
-        for (auto& l : s->lays) cells += (double)(l.ny + l.dn) * l.nxt;
-        if (g < 1 || RES_GRADIENT * us > STREAM_STEP_US + STREAM_CELL_US * cells) return FWI_OK;
+        for (auto& l : s->lays)
+            streaming += STREAM_CELL_US * l.ny * l.nx + STREAM_SIDE_US * 2 * l.dn * l.ny + STREAM_BOTTOM_US * l.dn * l.nxt;
+        if (g < 1 || RES_GRADIENT * us > streaming) return FWI_OK;
         const int nw = (D.nshots + g - 1) / g;
         g = (D.nshots + nw - 1) / nw;
         s->waves.clear();

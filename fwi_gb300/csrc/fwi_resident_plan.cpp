@@ -14,12 +14,11 @@ namespace {
 // ResGroup), and the modelled step in us: a fixed part (the barrier, the round
 // trip of the edges that the second phase does not hide), a part per pass over
 // the edge pairs, and the rows that the busiest threads march in either phase.
-// Measured while the computing threads still exchanged the edges: the steps
-// now take 0.3 (large tiles) to 1.1 us (small ones) less, much the same for
-// all cuts of a grid.  A model refitted to the present clocks chose cuts that
-// were 7 % faster on one 200 x 400 shot and 2-4 % slower on larger ones.
+// Within 15 % of the steps measured (1.7 to 6 us).  A model with the clocks
+// read in the kernel, phase by phase, chose cuts that were 7 % faster on one
+// 200 x 400 shot and 2-4 % slower on larger ones.
 constexpr double ROW_COST[4] = {1.0, 2.6, 1.3, 2.2};
-constexpr double STEP_US = 1.2, PAIR_US = 0.17, ROW_US[2] = {0.29, 0.21};
+constexpr double STEP_US = 0.4, PAIR_US = 0.17, ROW_US[2] = {0.29, 0.21};
 
 int ceil4(int v) { return (v + 3) / 4 * 4; }
 
