@@ -367,14 +367,14 @@ bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const
 
 int res_group(const std::vector<const Layout*>& lays, const ResDevice& dev, int max_shots, double* us_out) {
     const int n = (int)lays.size();
-    int best = 0;
+    int best = 0, equal = n - 1;  // equal: first shot of the run of equal widths that ends the list
+    while (equal > 0 && lays[equal - 1]->nx == lays[equal]->nx) --equal;
     double best_us = 0.0;
     for (int g = 1; g <= std::min(n, max_shots); ++g) {
         const int launches = (n + g - 1) / g, even = (n + launches - 1) / launches;
         if (even != g && g > 1) continue;  // another group size cuts the shots into as many launches
         double us = 0.0;
         for (int i = 0; i < n; i += g) {
-            // equal windows at both ends of the chunk: one model for runs of equal chunks
             const std::vector<const Layout*> part(lays.begin() + i, lays.begin() + std::min(n, i + g));
             const double t = best_form(part, dev, nullptr);
             if (t < 0) {
@@ -382,9 +382,11 @@ int res_group(const std::vector<const Layout*>& lays, const ResDevice& dev, int 
                 break;
             }
             us += t;
-            if (n - i >= 2 * g && lays[i]->nx == lays[n - 1]->nx) {  // equal widths all through (sorted)
-                us *= n / g;
-                i = n / g * g - g;
+            // equal widths from here on: the full launches that follow take the same time
+            if (i >= equal && n - i >= 2 * g) {
+                const int more = (n - i) / g - 1;
+                us += more * t;
+                i += more * g;
             }
         }
         if (us < 0) {
