@@ -2117,35 +2117,27 @@ int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
         std::vector<int> order(D.nshots);
         for (int i = 0; i < D.nshots; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return s->geoms[a].nx > s->geoms[b].nx; });
+        std::vector<const ShotGeom*> geoms;
         std::vector<const Layout*> lays;
-        for (int i : order) lays.push_back(&s->lays[i]);
-        double us = 0.0, streaming = STREAM_STEP_US;
-        int g = res_group(lays, L().res_dev, (int)most, &us);
+        for (int i : order) {
+            geoms.push_back(&s->geoms[i]);
+            lays.push_back(&s->lays[i]);
+        }
+        double streaming = STREAM_STEP_US;
         for (auto& l : s->lays)
             streaming += STREAM_CELL_US * l.ny * l.nx + STREAM_SIDE_US * 2 * l.dn * l.ny + STREAM_BOTTOM_US * l.dn * l.nxt;
-        if (g < 1 || RES_GRADIENT * us > streaming) return FWI_OK;
-        const int nw = (D.nshots + g - 1) / g;
-        g = (D.nshots + nw - 1) / nw;
+        ResSurvey plan;
+        bool fits = res_survey(geoms, lays, L().res_dev, (int)most, streaming / RES_GRADIENT, plan);
+        for (size_t w = 0; w < plan.launches.size() && fits; ++w) TRY(res_fits(plan.launches[w], D.acc, &fits));
+        if (!fits) return FWI_OK;
+        const int g = plan.shots;
         s->waves.clear();
         s->res.clear();
         size_t out = 0, c2 = 0;
         for (int i = 0; i < D.nshots; i += g) {
             s->waves.emplace_back(order.begin() + i, order.begin() + std::min(D.nshots, i + g));
-            std::vector<const ShotGeom*> geo;
-            std::vector<const Layout*> lay;
-            for (int sh : s->waves.back()) {
-                geo.push_back(&s->geoms[sh]);
-                lay.push_back(&s->lays[sh]);
-            }
             std::unique_ptr<ResDev> r(new ResDev());
-            ResCuts cuts;
-            bool fits = res_cuts(lay, L().res_dev, cuts) && res_plan(geo, lay, cuts, L().res_dev, r->plan);
-            if (fits) TRY(res_fits(r->plan, D.acc, &fits));
-            if (!fits) {
-                s->waves.clear();
-                s->res.clear();
-                return FWI_OK;
-            }
+            r->plan = std::move(plan.launches[i / g]);
             TRY(res_upload(*r, st));
             out = std::max(out, r->plan.out_elems);
             c2 = std::max(c2, r->plan.c2_elems);

@@ -106,10 +106,12 @@ struct ResCuts {
     double step_us = 0.0;    // modelled time of one step
 };
 
-// Cut the shots of a launch; false when they do not fit the device together.
-bool res_cuts(const std::vector<const Layout*>& lays, const ResDevice& dev, ResCuts& out);
-// Plan a launch for the shots (geoms[i], lays[i]) with their cuts; false when
-// a tile's sources and receivers do not fit beside it.
+// Cut the shots of a launch, c2 in shared memory where they fit with it (and
+// c2_shared allows it); false when they do not fit the device together.
+bool res_cuts(const std::vector<const Layout*>& lays, const ResDevice& dev, ResCuts& out, bool c2_shared = true);
+// Plan a launch for the shots (geoms[i], lays[i]) with their cuts, or, where a
+// tile's sources and receivers do not fit beside its c2, with cuts that keep
+// c2 in global memory; false when they do not fit there either.
 bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResCuts& cuts,
               const ResDevice& dev, ResPlan& out);
 
@@ -117,5 +119,17 @@ bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const
 // groups of at most max_shots) with the smallest modelled time; 0 when some
 // shot does not fit.  *us: that time, per step of all shots.
 int res_group(const std::vector<const Layout*>& lays, const ResDevice& dev, int max_shots, double* us = nullptr);
+
+// The launches of a survey, over its shots in the given order.
+struct ResSurvey {
+    int shots = 0;                  // per launch
+    double us = 0.0;                // modelled time of a step of all shots
+    std::vector<ResPlan> launches;
+};
+// The shots per launch that res_group chooses, or the next smaller choice whose
+// launches hold their sources and receivers (the cuts are made for the grids
+// alone); false when no choice within limit_us does.
+bool res_survey(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResDevice& dev,
+                int max_shots, double limit_us, ResSurvey& out);
 
 }  // namespace fwi

@@ -284,9 +284,10 @@ double model(const std::vector<const Layout*>& lays, const ResDevice& dev, bool 
     return t;
 }
 
-// c2 in shared memory where the shots fit with it, else in global memory.
-double best_form(const std::vector<const Layout*>& lays, const ResDevice& dev, bool* c2_shared) {
+// c2 in shared memory where the shots fit with it (and it may be), else in global memory.
+double best_form(const std::vector<const Layout*>& lays, const ResDevice& dev, bool* c2_shared, bool may_share = true) {
     for (const bool c2 : {true, false}) {
+        if (c2 && !may_share) continue;
         const double t = model(lays, dev, c2, nullptr);
         if (t < 0) continue;
         if (c2_shared) *c2_shared = c2;
@@ -295,17 +296,10 @@ double best_form(const std::vector<const Layout*>& lays, const ResDevice& dev, b
     return -1.0;
 }
 
-}  // namespace
-
-bool res_cuts(const std::vector<const Layout*>& lays, const ResDevice& dev, ResCuts& out) {
-    out = ResCuts();
-    if (best_form(lays, dev, &out.c2_shared) < 0) return false;
-    out.step_us = model(lays, dev, out.c2_shared, &out.shots);
-    return true;
-}
-
-bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResCuts& cuts,
-              const ResDevice& dev, ResPlan& out) {
+// A launch with the given cuts; false when a tile's sources and receivers do
+// not fit beside it.
+bool plan_cuts(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResCuts& cuts,
+               const ResDevice& dev, ResPlan& out) {
     out = ResPlan();
     out.c2_shared = cuts.c2_shared;
     const size_t cap = smem_cap(dev);
@@ -365,6 +359,22 @@ bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const
     return (int)out.tiles.size() <= dev.sms;
 }
 
+}  // namespace
+
+bool res_cuts(const std::vector<const Layout*>& lays, const ResDevice& dev, ResCuts& out, bool c2_shared) {
+    out = ResCuts();
+    if (best_form(lays, dev, &out.c2_shared, c2_shared) < 0) return false;
+    out.step_us = model(lays, dev, out.c2_shared, &out.shots);
+    return true;
+}
+
+bool res_plan(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResCuts& cuts,
+              const ResDevice& dev, ResPlan& out) {
+    if (plan_cuts(geoms, lays, cuts, dev, out)) return true;
+    ResCuts global;
+    return cuts.c2_shared && res_cuts(lays, dev, global, false) && plan_cuts(geoms, lays, global, dev, out);
+}
+
 int res_group(const std::vector<const Layout*>& lays, const ResDevice& dev, int max_shots, double* us_out) {
     const int n = (int)lays.size();
     int best = 0, equal = n - 1;  // equal: first shot of the run of equal widths that ends the list
@@ -400,6 +410,27 @@ int res_group(const std::vector<const Layout*>& lays, const ResDevice& dev, int 
     }
     if (us_out) *us_out = best_us;
     return best;
+}
+
+bool res_survey(const std::vector<const ShotGeom*>& geoms, const std::vector<const Layout*>& lays, const ResDevice& dev,
+                int max_shots, double limit_us, ResSurvey& out) {
+    const int n = (int)lays.size();
+    for (int most = max_shots; most >= 1; most = out.shots - 1) {
+        out = ResSurvey();
+        out.shots = res_group(lays, dev, most, &out.us);
+        if (out.shots < 1 || out.us > limit_us) return false;
+        bool fits = true;
+        for (int i = 0; i < n && fits; i += out.shots) {
+            const int e = std::min(n, i + out.shots);
+            const std::vector<const Layout*> part(lays.begin() + i, lays.begin() + e);
+            ResCuts cuts;
+            out.launches.emplace_back();
+            fits = res_cuts(part, dev, cuts) &&
+                   res_plan({geoms.begin() + i, geoms.begin() + e}, part, cuts, dev, out.launches.back());
+        }
+        if (fits) return true;
+    }
+    return false;
 }
 
 }  // namespace fwi
