@@ -507,7 +507,8 @@ def main():
 
     # roofline of the dominant kernel pair (main + bottom step kernels)
     hbm, peak_kind = peaks()
-    nsteps = 200
+    # (a resident survey's call waits for its launches: enough steps that the wait does not show)
+    nsteps = 2000 if sv.resident() else 200
     sv.time_steps(20)
     torch.cuda.synchronize()
     r0, r1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -2753,16 +2753,21 @@ namespace {
 int time_wave0_steps(fwi_survey* s, int steps, float* ms, bool single_only) {
     const auto& D = s->desc;
     if (s->resident) {  // launches of at most nt-1 steps, each from a state at rest
+        int* word = reinterpret_cast<int*>(s->d_mis_tr.as<double>() + s->ntr);
+        int err = 0;
+        CK(cudaMemsetAsync(word, 0, sizeof err, stream()));
         for (int n; steps > 0; steps -= n) {
             n = std::min(steps, D.nt - 1);
             ResParams p = res_params(*s->res[0], 0, D.acc, D.dt, D.d, D.nt, D.store_snap, s->nt_store, D.grad_form,
-                                     s->d_fA, s->d_fB, s->res_out, s->res_c2,
-                                     reinterpret_cast<int*>(s->d_mis_tr.as<double>() + s->ntr));
+                                     s->d_fA, s->d_fB, s->res_out, s->res_c2, word);
             p.from_lambda = 1;
             p.steps = n + 1;
             TRY(res_launch(*s->res[0], D.acc, 0, p, stream()));
         }
-        return FWI_OK;
+        // a launch that gave up a wait ends early: its time is no step's time
+        CK(cudaMemcpyAsync(&err, word, sizeof err, cudaMemcpyDeviceToHost, stream()));
+        CK(cudaStreamSynchronize(stream()));
+        return res_error(err);
     }
     auto& wd = *s->wdev[0];
     StepSet ps;

@@ -351,7 +351,8 @@ int fwi_survey_launch_form(fwi_survey* s, int step, int* form, float* direct_ms,
 int fwi_survey_recompute(fwi_survey* s, int* segment_steps, int* segments);
 /* Run `steps` forward time steps of the first wave (for kernel timing; the
  * wavefields keep evolving, sources are injected; a resident survey starts
- * from rest). */
+ * from rest, and its call waits for the launches to learn whether they ended
+ * early). */
 int fwi_survey_time_steps(fwi_survey* s, int steps);
 
 /* calculate_misfit_gradient(iter,step,f1,f2,dt,nt,tfin,S0,Misfit,Grad) for
