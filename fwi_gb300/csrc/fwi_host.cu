@@ -1324,6 +1324,8 @@ struct fwi_survey {
     std::vector<std::unique_ptr<ResDev>> res;
     DBuf res_out, res_c2;
     std::unique_ptr<fwi_survey> streaming;
+    const fwi_survey* plan_of = nullptr;  // of a streaming plan in the making: its resident survey
+    bool planned = true;                  // of a streaming plan: timed (its fields fitted the device)
     // checkpointed recomputation: C forward steps per segment, J segments,
     // `slots` snapshot blocks per shot; per block its segment and slot
     int rc_C = 0, rc_J = 0, rc_slots = 0;
@@ -1378,7 +1380,8 @@ int survey_prepare_slots(fwi_survey* s) {
                 big = l;
             }
         }
-        TRY(s->slots[k]->alloc(big, s->rc_C ? s->rc_slots : s->nt_store + 1, D.snap_form, D.grad_form));
+        // (a plan of a resident survey is timed over forward steps alone: no snapshots)
+        TRY(s->slots[k]->alloc(big, s->rc_C ? s->rc_slots : s->plan_of ? 1 : s->nt_store + 1, D.snap_form, D.grad_form));
         if (s->rc_C) TRY(s->slots[k]->alloc_rc(s->rc_J - 1));
     }
     return FWI_OK;
@@ -2203,8 +2206,9 @@ int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
 int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
     const auto& D = s->desc;
     s->rc_C = 0;
+    const fwi_survey& own = s->plan_of ? *s->plan_of : *s;  // the survey that holds the data
     size_t held = 0;
-    for (auto& sl : s->slots) held += sl->bytes();
+    for (auto& sl : own.slots) held += sl->bytes();
     // wave size from the HBM budget
     size_t per = 0;
     for (auto& l : s->lays) per = std::max(per, shot_wave_bytes(l, s->nt_store, D.snap_form, D.grad_form));
@@ -2212,7 +2216,7 @@ int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
     CK(cudaMemGetInfo(&freeb, &totb));
     size_t budget = (size_t)(0.92 * (double)(freeb + held));
     if (s->desc.hbm_budget) {
-        size_t used_resident = s->d_obs.n + s->d_synth.n + s->d_adj.n + s->d_src.n + s->d_G.n + s->d_lambda.n;
+        size_t used_resident = own.d_obs.n + own.d_synth.n + own.d_adj.n + own.d_src.n + own.d_G.n + own.d_lambda.n;
         if (s->desc.hbm_budget <= used_resident) return fail(FWI_ERR_NOMEM, "HBM budget smaller than the resident data");
         budget = std::min(budget, s->desc.hbm_budget - used_resident);
     }
@@ -2248,7 +2252,7 @@ int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
             if (wave_rc < 1)
                 return fail(FWI_ERR_NOMEM, "one shot's checkpoints and snapshot ring (" + std::to_string(per_rc) +
                                                " bytes) exceed the device budget");
-            TRY(rc_plan(s, C));
+            if (!s->plan_of) TRY(rc_plan(s, C));
             wave = wave_rc;
         }
     }
@@ -2266,25 +2270,24 @@ int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
     return survey_prepare_waves(s);
 }
 
-// The survey whose streaming plan and tuning answer the query entries: *s
-// itself, or, for a resident survey, a plan of the streaming kernels for the
-// same shots, made (and tuned) on the first query; its fields are freed again.
-int streaming_view(fwi_survey** sp) {
-    fwi_survey* s = *sp;
-    if (!s->resident) return FWI_OK;
-    if (!s->streaming) {
-        std::unique_ptr<fwi_survey> c(new fwi_survey());
-        c->desc = s->desc;
-        c->nt_store = s->nt_store;
-        c->geoms = s->geoms;
-        c->lays = s->lays;
-        c->gw = s->gw;
-        c->mw = s->mw;
-        c->tr_off = s->tr_off;
-        c->ntr = s->ntr;
-        c->h_fA = s->h_fA;
-        c->h_fB = s->h_fB;
+// A resident survey's plan of the streaming kernels for the same shots: the
+// waves that they would run, timed over forward steps (tuned) or not.
+int streaming_plan(fwi_survey* s, bool tuned, std::unique_ptr<fwi_survey>& out) {
+    std::unique_ptr<fwi_survey> c(new fwi_survey());
+    c->desc = s->desc;
+    c->nt_store = s->nt_store;
+    c->geoms = s->geoms;
+    c->lays = s->lays;
+    c->gw = s->gw;
+    c->mw = s->mw;
+    c->tr_off = s->tr_off;
+    c->ntr = s->ntr;
+    c->h_fA = s->h_fA;
+    c->h_fB = s->h_fB;
+    c->planned = tuned;
+    if (tuned) {
         cudaStream_t st = stream();
+        c->plan_of = s;
         TRY(upload(c->d_fA, c->h_fA, st));
         TRY(upload(c->d_fB, c->h_fB, st));
         TRY(c->d_src.alloc(s->d_src.n));
@@ -2292,10 +2295,33 @@ int streaming_view(fwi_survey** sp) {
         TRY(c->d_adj.alloc(16));
         CK(cudaMemsetAsync(c->d_src.p, 0, c->d_src.n, st));
         TRY(survey_plan(c.get(), true, true));
+        c->plan_of = nullptr;
         c->slots.clear();
         c->d_src.release();
         c->d_synth.release();
-        s->streaming = std::move(c);
+    } else {
+        c->wdev.emplace_back(new fwi_survey::WaveDev());
+        for (auto& l : c->lays) c->wdev[0]->n_ff += two_step_ok(l);
+    }
+    out = std::move(c);
+    return FWI_OK;
+}
+
+// The survey whose streaming plan and tuning answer the query entries: *s
+// itself, or, for a resident survey, its streaming plan, made (and tuned) on
+// the first query; its fields are freed again.  Where they do not fit beside
+// the survey, or within its budget, the plan before any tuning answers: a
+// query does not fail for memory that the survey itself does not need.
+int streaming_view(fwi_survey** sp) {
+    fwi_survey* s = *sp;
+    if (!s->resident) return FWI_OK;
+    if (!s->streaming || !s->streaming->planned) {
+        int rc = streaming_plan(s, true, s->streaming);
+        if (rc == FWI_ERR_NOMEM) {
+            cudaGetLastError();  // of the refused allocation
+            rc = streaming_plan(s, false, s->streaming);
+        }
+        TRY(rc);
     }
     *sp = s->streaming.get();
     return FWI_OK;
