@@ -1330,6 +1330,20 @@ struct fwi_survey {
     // `slots` snapshot blocks per shot; per block its segment and slot
     int rc_C = 0, rc_J = 0, rc_slots = 0;
     std::vector<int> ev, blk_seg, blk_slot;
+    // the tuner's choices and timings of another plan for the same shots
+    void take_tuning(const fwi_survey& o) {
+        band = o.band;
+        tile_var = o.tile_var;
+        tile_band = o.tile_band;
+        tile_eband = o.tile_eband;
+        single_step = o.single_step;
+        fused = o.fused;
+        tune_two_ms = o.tune_two_ms;
+        tune_single_ms = o.tune_single_ms;
+        tune_fused_ms = o.tune_fused_ms;
+        tune_ms = o.tune_ms;
+        tune_ems = o.tune_ems;
+    }
     ~fwi_survey() {
         if (obs_ready) cudaEventDestroy(obs_ready);
         for (auto& w : wdev) {
@@ -2194,7 +2208,6 @@ int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
     }
     CK(cudaStreamSynchronize(st));
     s->resident = true;
-    s->streaming.reset();
     *ok = true;
     return FWI_OK;
 }
@@ -2224,7 +2237,11 @@ int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
         bool res = false;
         TRY(resident_plan(s, budget, &res));
         if (res) return FWI_OK;
-        if (s->resident) tune = true;  // a longer time axis no longer fits: the first streaming plan
+        if (s->resident) {  // a longer time axis no longer fits: the tuning that its queries gave, or a first one
+            if (s->streaming && s->streaming->planned) s->take_tuning(*s->streaming);
+            else tune = s->tune_ms.empty();
+        }
+        s->streaming.reset();
         s->resident = false;
         s->res.clear();
     }
@@ -2271,7 +2288,8 @@ int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
 }
 
 // A resident survey's plan of the streaming kernels for the same shots: the
-// waves that they would run, timed over forward steps (tuned) or not.
+// waves that they would run, timed over forward steps (tuned) or not.  It
+// outlives a change of the time axis, as a streaming survey's tuning does.
 int streaming_plan(fwi_survey* s, bool tuned, std::unique_ptr<fwi_survey>& out) {
     std::unique_ptr<fwi_survey> c(new fwi_survey());
     c->desc = s->desc;
@@ -2294,7 +2312,8 @@ int streaming_plan(fwi_survey* s, bool tuned, std::unique_ptr<fwi_survey>& out) 
         TRY(c->d_synth.alloc(s->d_synth.n));
         TRY(c->d_adj.alloc(16));
         CK(cudaMemsetAsync(c->d_src.p, 0, c->d_src.n, st));
-        TRY(survey_plan(c.get(), true, true));
+        if (!s->tune_ms.empty()) c->take_tuning(*s);  // tuned on a time axis that it streamed
+        TRY(survey_plan(c.get(), s->tune_ms.empty(), true));
         c->plan_of = nullptr;
         c->slots.clear();
         c->d_src.release();

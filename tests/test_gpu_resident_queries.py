@@ -1,6 +1,7 @@
 """The tuning queries of a resident survey (tiles, edge_tiles, stepping, tuning):
 they answer where the streaming kernels' fields do not fit the survey's budget,
-and leave the survey as it was."""
+leave the survey as it was, and keep their timings on another time axis, also
+where the survey leaves the resident kernel and comes back."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,52 @@ def test_queries_within_a_budget_too_small_for_the_streaming_plan():
     g2 = np.zeros_like(g)
     assert sv.run(1, g2)[0] == m and np.array_equal(g2, g)
     sv.close()
+
+
+def test_timings_outlive_a_new_time_axis(monkeypatch):
+    monkeypatch.setenv("FWI_TUNE_CACHE", "")  # no cross-process cache file
+    import fwi_gb300 as F
+    from fwi_gb300 import synth
+    spec, vp = synth.small_survey(seed=52, ny=61, nxm=307, nshots=2, dpml=20, nt=60)
+    lam = synth.lam_from_vp(vp)
+    rng = np.random.default_rng(7)
+    nrec = sum(len(s.nxRec) for s in spec.shots)
+    nsou = sum(len(s.nxSou) for s in spec.shots)
+
+    def axis(nt):
+        return (1e-3, nt, rng.standard_normal(nt * nsou).astype(np.float32), rng.standard_normal(nt * nrec).astype(np.float32))
+
+    # the budget holds the streaming state of both shots at 800 steps, their resident images (12 bytes a cell and
+    # 4 a snapshot) up to some 2000 steps, and the streaming state with checkpoints above that
+    cells = spec.ny * 512
+    data = 4 * 6000 * (3 * nrec + nsou) + 12 * spec.ny * spec.nx_model
+    sv = F.Survey(spec, hbm_budget=data + 2 * cells * (12 + 4 * 200))
+    assert sv.resident() == 2
+    first = queries(sv)
+    assert first[0][2] and first[2][1]  # timed on the first query
+    sv.set_time(*axis(80))
+    assert sv.resident() == 2 and queries(sv) == first
+    long = axis(6000)
+    sv.set_time(*long)
+    assert sv.resident() == 0
+    away = queries(sv)
+    assert away[0][2] == first[0][2] and away[2] == first[2]
+    sv.set_lambda(lam)
+    g = np.zeros((spec.ny, spec.nx_model), np.float32, order="F")
+    m, _ = sv.run(1, g)
+    short = axis(80)
+    sv.set_time(*short)
+    assert sv.resident() == 2 and queries(sv) == first
+    ms, _ = sv.run(2)
+    sv.close()
+    # either axis from a survey that streams from the start
+    for (dt, nt, src, obs), want in ((long, m), (short, ms)):
+        ref = F.Survey(spec, two_step=False)
+        ref.set_time(dt, nt, src, obs)
+        ref.set_lambda(lam)
+        g2 = np.zeros_like(g)
+        m2, _ = ref.run(1, g2)
+        assert m2 == want
+        if nt == 6000:
+            np.testing.assert_array_equal(g2, g)
+        ref.close()
