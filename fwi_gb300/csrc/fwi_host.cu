@@ -2218,7 +2218,7 @@ int resident_plan(fwi_survey* s, size_t budget, bool* ok) {
 // buffers only grow), the band height and the work lists of every wave.
 int survey_plan(fwi_survey* s, bool tune, bool streaming = false) {
     const auto& D = s->desc;
-    s->rc_C = 0;
+    s->rc_C = s->rc_J = 0;
     const fwi_survey& own = s->plan_of ? *s->plan_of : *s;  // the survey that holds the data
     size_t held = 0;
     for (auto& sl : own.slots) held += sl->bytes();

@@ -61,7 +61,7 @@ def test_timings_outlive_a_new_time_axis(monkeypatch):
     assert sv.resident() == 2 and queries(sv) == first
     long = axis(6000)
     sv.set_time(*long)
-    assert sv.resident() == 0
+    assert sv.resident() == 0 and sv.recompute_plan()[1] > 1
     away = queries(sv)
     assert away[0][2] == first[0][2] and away[2] == first[2]
     sv.set_lambda(lam)
@@ -70,6 +70,7 @@ def test_timings_outlive_a_new_time_axis(monkeypatch):
     short = axis(80)
     sv.set_time(*short)
     assert sv.resident() == 2 and queries(sv) == first
+    assert sv.recompute_plan() == (0, 0)
     ms, _ = sv.run(2)
     sv.close()
     # either axis from a survey that streams from the start
