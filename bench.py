@@ -32,6 +32,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "shot-gradients/s"
+# beside the tuner's fields of a resident survey
+STREAMING_PLAN = ("band, tile, tuner and time_stepping fields describe the streaming kernels' plan for the same shots, "
+                  "which this run does not use")
 
 
 def parse():
@@ -549,7 +552,11 @@ def main():
             "two_step_tile_bytes_per_pass": tile_bytes_pass,
             "peak_kind": f"{peak_kind} copy bandwidth (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
             else "fallback 6.8 TB/s"}
-    if a.workload == "single":
+    if resident:
+        roof["note"] = ("the wave's state stays in shared memory, so HBM does not bound the step: frac is the rate at which "
+                        "a streaming step would have to run to take as long, and may exceed 1; the row loops are bound "
+                        "by FP32 issue and shared-memory bandwidth, small grids by the exchange of the tile edges")
+    elif a.workload == "single":
         roof["note"] = ("one 200x400 shot: its wavefields (10 x 256 x 512 floats = 5 MB) stay in the 129 MB L2, "
                         "so the step is latency-bound and its fraction of the HBM peak is not meaningful")
     sv.close()
@@ -576,7 +583,9 @@ def main():
         torch.cuda.synchronize()
         tp = p0.elapsed_time(p1) / 1e3 / nplain
         plain = {"value": 1.0 / tp, "unit": METRIC, "batched_over_plain": value / world * tp,
-                 "how": "same workload one shot at a time, direct kernel launches, no CUDA graph"}
+                 "how": "same workload one shot at a time, direct launches of the streaming kernels, no CUDA graph"
+                 + ("; the batched run is resident, so the ratio compares the two kernels as well as the batching"
+                    if resident else "")}
         pv.close()
         del pv
         torch.cuda.synchronize()
@@ -635,9 +644,11 @@ def main():
         batch_plan = None
         if bsv is not None:
             bk, br, _ = bsv.tiles()
-            batch_plan = {"tile_kernel": bk, "tile_rows": br, "tile_edge_rows": bsv.edge_tiles()[0],
+            batch_plan = {"resident_shots_per_launch": bsv.resident(), "tile_kernel": bk, "tile_rows": br,
+                          "tile_edge_rows": bsv.edge_tiles()[0],
                           "wave_band": list(bsv.tuning()), "time_stepping": bsv.stepping()[0],
-                          "launch": list(bsv.launch_form(1))}
+                          "launch": list(bsv.launch_form(1)),
+                          "note": STREAMING_PLAN if bsv.resident() else None}
         e2e = {"value": world * len(spec.shots) * a.steps / te, "unit": METRIC,
                "h2d_bytes_per_step": int(h_lam.nbytes + h_obs.nbytes + h_src.nbytes + h_grad.nbytes),
                "d2h_bytes_per_step": int(h_grad.nbytes + 8 * sum(len(s.nxRec) for s in spec.shots)),
@@ -652,6 +663,12 @@ def main():
         cpu = {"value": rate, "unit": METRIC, "cores": nthreads, "kind": "port", "sample": desc,
                "seconds": tcpu}
 
+    l2 = "inputs larger than L2 (wavefields of all shots of a wave and their snapshots: tens to hundreds of GB)"
+    if resident:
+        mb = sum(sorted(4e-6 * (spec.nt_store + 1) * spec.ny * sh.nx for sh in spec.shots)[-resident:])
+        l2 = (f"state in shared memory; the snapshots of a launch's shots, {mb:.0f} MB, are written by its forward and "
+              f"read by its adjoint pass ({'larger' if mb > 129 else 'smaller'} than the 129 MB L2, not flushed)")
+
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": a.steps,
                 "warmup": a.warmup, "ms_per_step": t / a.steps * 1e3, "higher_is_better": True, "scaling": "weak",
@@ -663,12 +680,13 @@ def main():
                            "tuner_ms_per_pass": {f"{k}/{r}": v for (k, r), v in tile_ms.items()},
                            "tuner_edge_ms_per_pass": {str(k): v for k, v in edge_ms.items()},
                            "resident_shots_per_launch": resident,
+                           "kernel": "k_resident" if resident else "streaming",
+                           "streaming_plan": STREAMING_PLAN if resident else None,
                            "recompute_segment_steps": rc_plan[0], "recompute_segments": rc_plan[1],
                            "launch": {"form": launch_form, "direct_ms": launch_direct_ms,
                                       "graph_replay_ms": launch_graph_ms},
                            "time_stepping": {"form": stepping, "tuner_ms_per_2_steps": stepping_ms},
-                           "l2": "inputs larger than L2 (wavefields of all shots of a wave and their snapshots: "
-                                 "tens to hundreds of GB)"},
+                           "l2": l2},
                 "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "plain": plain, "gpu_launches": int(launches),
                 "clocks": clk}
         print(json.dumps(line), flush=True)
