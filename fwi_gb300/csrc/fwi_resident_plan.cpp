@@ -12,11 +12,16 @@ namespace {
 
 // Cost of one row of a thread's work relative to interior quads (the kinds of
 // ResGroup), and the modelled step in us: a fixed part (the barrier, the round
-// trip of the edges that the second phase does not hide), a part per pass over
-// the edge pairs, and the rows that the busiest threads march in either phase.
-// Within 15 % of the steps measured (1.7 to 6 us).  A model with the clocks
-// read in the kernel, phase by phase, chose cuts that were 7 % faster on one
-// 200 x 400 shot and 2-4 % slower on larger ones.
+// trip of the edges that the second phase does not hide), a part per RES_THREADS
+// edge pairs (a fit: the kernel's own passes are RES_COMM threads times one to
+// RES_WORDS pairs), and the rows that the busiest threads march in either phase.
+// Against measured forward steps, modelled / measured in us: three shots of
+// 400 x 2000 5.06 / 4.97 (8th order 5.06 / 5.77), 600 x 4000 4.43 / 4.26, five
+// of 600 x 812 5.79 / 5.20, five of 251 x 1013 3.70 / 3.32, twelve of 163 x 384
+// 3.32 / 2.84, one of 200 x 400 2.13 / 1.73, three of 40 x 90 1.67 / 1.43; with
+// deep pads (dpml 40 to 50) 19 to 38 % high.  A model with the clocks read in
+// the kernel, phase by phase, chose cuts that were 7 % faster on one 200 x 400
+// shot and 2-4 % slower on larger ones.
 constexpr double ROW_COST[4] = {1.0, 2.6, 1.3, 2.2};
 constexpr double STEP_US = 0.4, PAIR_US = 0.17, ROW_US[2] = {0.29, 0.21};
 

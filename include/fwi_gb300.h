@@ -313,10 +313,13 @@ int fwi_survey_two_step_bytes(fwi_survey* s, double* per_step, double* tiles_per
  * with their state in shared memory (the first wave's; the default where it is
  * modelled faster, the shots fit and the snapshots are FP32); 0: the survey
  * runs the streaming kernels.  The tuning entries below describe the streaming
- * kernels' plan for the same shots (made when first asked for): what the
- * survey would run with one of their forms asked for in the descriptor. */
+ * kernels' plan for the same shots (made and timed when first asked for; where
+ * its fields do not fit the device or the budget, the plan before any tuning,
+ * with no timings): what the survey would run with one of their forms asked
+ * for in the descriptor. */
 int fwi_survey_resident(fwi_survey* s, int* shots_per_launch);
-/* Tuning chosen for the survey (wave size, band rows). */
+/* Tuning chosen for the survey (wave size -- of a resident survey its shots
+ * per launch -- and band rows). */
 int fwi_survey_tuning(fwi_survey* s, int* wave_shots, int* band_rows);
 /* Two-step tiles chosen for the survey: kernel (1 = register queues, 2 =
  * shared-memory queue; 0 when the survey runs single steps only) and rows per
